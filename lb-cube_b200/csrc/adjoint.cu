@@ -138,7 +138,8 @@ struct GradientLayout {
   size_t field;      // bytes of one population field
   long long ckpts;   // checkpoints stored (including the initial state)
   size_t off_ckpt, off_seg, off_lam, off_slots, total;
-  long long slots;   // FP64 slots (blocks)
+  long long slots;   // FP64 slots (room for every block)
+  long long used;    // slots that the launches write
 };
 
 inline GradientLayout gradient_layout(int Q, size_t elem, const Grid& g, int steps, int interval) {
@@ -147,6 +148,7 @@ inline GradientLayout gradient_layout(int Q, size_t elem, const Grid& g, int ste
   l.field = (l.field + 255) / 256 * 256;
   l.ckpts = (steps + interval - 1) / interval + 1;
   l.slots = g.blocks();
+  l.used = g.launched();
   l.off_ckpt = 0;
   l.off_seg = l.off_ckpt + (size_t)l.ckpts * l.field;
   l.off_lam = l.off_seg + (size_t)interval * l.field;
@@ -217,8 +219,8 @@ cudaError_t ke_gradient(int collision, const Real* rho0, const Real* u0, const G
   }
   velocity_gradient_kernel<L, Real><<<grid_dims(g), block_dims(g), 0, s>>>(rho0, u0, lam[0], grad_u0, g);
   if ((err = cudaGetLastError()) != cudaSuccess) return err;
-  sum_slots_kernel<<<1, 1024, 0, s>>>(ke_slots, lay.slots, 1, 1.0, out);
-  sum_slots_kernel<<<1, 1024, 0, s>>>(dtau_slots, lay.slots, 1, 1.0, out + 1);
+  sum_slots_kernel<<<1, 1024, 0, s>>>(ke_slots, lay.used, 1, 1.0, out);
+  sum_slots_kernel<<<1, 1024, 0, s>>>(dtau_slots, lay.used, 1, 1.0, out + 1);
   return cudaGetLastError();
 }
 

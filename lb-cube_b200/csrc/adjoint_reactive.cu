@@ -667,9 +667,9 @@ cudaError_t reactive_gradient(int collision, int objective, const Real* rho0, co
         cudaSuccess)
       return err;
   } else {
-    sum_slots_kernel<<<1, 1024, 0, s>>>(j_slots, lay.blocks, 1, 1.0 / (double)g.plane, out);
+    sum_slots_kernel<<<1, 1024, 0, s>>>(j_slots, g.launched(), 1, 1.0 / (double)g.plane, out);
   }
-  const long long nslots = lay.blocks * kWarpsPerBlock;
+  const long long nslots = g.launched() * kWarpsPerBlock;
   sum_slots_kernel<<<1, 1024, 0, s>>>(slots + 0, nslots, kReactiveSlots, 1.0, out + 1);
   sum_slots_kernel<<<1, 1024, 0, s>>>(slots + 1, nslots, kReactiveSlots, 1.0, out + 2);
   sum_slots_kernel<<<1, 1024, 0, s>>>(slots + 2, nslots, kReactiveSlots, -omega_c * omega_c,
@@ -1173,8 +1173,8 @@ extern "C" int lbm_reactive_slab_sums_async(int fluid_lattice, size_t x_extent, 
   if (slots_bytes < slab_slots_bytes(g) || partials_bytes < (size_t)g.blocks() * sizeof(double))
     return (int)cudaErrorInvalidValue;
   const cudaStream_t s = as_stream(stream);
-  const long long nslots = g.blocks() * kWarpsPerBlock;
-  sum_slots_kernel<<<1, 1024, 0, s>>>(objective_partials, g.blocks(), 1, 1.0, sums);
+  const long long nslots = g.launched() * kWarpsPerBlock;
+  sum_slots_kernel<<<1, 1024, 0, s>>>(objective_partials, g.launched(), 1, 1.0, sums);
   for (int k = 0; k < kReactiveSlots; ++k)
     sum_slots_kernel<<<1, 1024, 0, s>>>(slots + k, nslots, kReactiveSlots, 1.0, sums + 1 + k);
   return (int)cudaGetLastError();

@@ -119,7 +119,7 @@ cudaError_t launch_diagnostics(const void* vf, size_t nx, size_t ny, size_t nz, 
   if (any_overlap(reads, writes)) return cudaErrorInvalidValue;
   err = launch_pdl(diag_partials_kernel<L, Real>, grid_dims(g), dim3(block_dims(g)), 0, s, f, g, partials);
   if (err != cudaSuccess) return err;
-  return launch_diag_finalize(partials, g.blocks(), speed_limit, out, s);
+  return launch_diag_finalize(partials, g.launched(), speed_limit, out, s);
 }
 
 template <class Real>

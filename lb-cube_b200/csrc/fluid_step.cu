@@ -75,7 +75,7 @@ cudaError_t launch_fluid_step_diag(const Real* cur, Real* nxt, size_t nx, size_t
     }
   }
   if (count < 0) {
-    count = g.blocks();
+    count = g.launched();
     err = launch_pdl(fluid_step_kernel<L, Real, CT, true>, grid_dims(g), dim3(block_dims(g)), 0, stream, cur,
                      nxt, g, omega, omega_minus, partials);
   }
