@@ -319,21 +319,17 @@ int lbm_reactive_stats_async(int scalar_lattice, int precision, const void* curr
  * the values themselves, so the step is deterministic); conversions and the
  * other paths round to nearest. Buffers are uint16 [Q, Z, Y, X]; x_extent
  * must be a multiple of 4 and buffers 8-byte aligned (else
- * cudaErrorInvalidValue). rho0 is the reference density of the shift. With
- * x_extent a multiple of 8 (at most 1024) and 16-byte aligned buffers, the
- * D2Q9 / D3Q19 BGK, TRT and MRT steps stage each row's source rows in shared
- * memory with bulk copies (see lbm_stage_timeouts).
+ * cudaErrorInvalidValue). rho0 is the reference density of the shift.
  * ------------------------------------------------------------------------- */
 int lbm_step_shifted_async(int lattice, int format, int collision,
     const void* current_populations, void* next_populations, size_t x_extent,
     size_t y_extent, size_t z_extent, float omega, float rho0, void* stream);
 
-/* Blocks of the row-staged 16-bit step (no reference counterpart) that gave
- * up waiting for a shared-memory row copy, since the count was last reset, on
- * the current device; every wait in that kernel is bounded, so a copy that
- * never lands ends the launch with this count raised instead of hanging it.
- * `reset` non-zero clears the count. Synchronous; returns 0xFFFFFFFF if the
- * count cannot be read. */
+/* Blocks of the 16-bit step (no reference counterpart) that gave up waiting
+ * for a copy of their inputs. The step reads its inputs with plain loads, so
+ * the count is always 0, whatever `reset`; the call still waits for the work
+ * on the legacy default stream and returns 0xFFFFFFFF if that reports an
+ * error. */
 unsigned int lbm_stage_timeouts(int reset);
 
 /* FP32/FP64 populations (`precision`) -> shifted 16-bit form, any lattice

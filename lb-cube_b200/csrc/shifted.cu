@@ -3,43 +3,28 @@
 //
 // An extension with no reference counterpart. Populations are stored as codes
 // of v_i = S (f_i / w_i - rho0) in 16 bits (collide_dev.cuh), halving the bytes
-// per lattice update (D3Q19: 76 B instead of 152 B). BGK and TRT collide on
-// the deviations v directly (DevStorage); MRT and RLBM decode to f, run the
-// reference operator and re-encode (ShiftedStorage). Rounding to 16 bits is to
-// nearest. Encode/decode kernels convert between FP32/FP64 populations and the
-// 16-bit form.
+// per lattice update (D3Q19: 76 B instead of 152 B). BGK, TRT and the D2Q9 /
+// D3Q19 MRT collide on the deviations v directly (DevStorage); RLBM and the
+// D3Q27 MRT decode to f, run the reference operator and re-encode
+// (ShiftedStorage). The step kernel is stream_codes.cuh. Encode/decode kernels
+// convert between FP32/FP64 populations and the 16-bit form, to nearest.
 #include <algorithm>
 #include <type_traits>
 
 #include "collide.cuh"
 #include "common.cuh"
-#include "stream_staged.cuh"
+#include "stream_codes.cuh"
 #include "stream_vec.cuh"
 #include "../../include/lbcube_b200.h"
 
 namespace lbcube {
-
-// Cells per thread of the 16-bit kernels: four (8-byte words of codes).
-#ifndef LBCUBE_SHIFTED_CELLS
-#define LBCUBE_SHIFTED_CELLS 4
-#endif
-template <int FMT>
-constexpr int kShiftedCells = LBCUBE_SHIFTED_CELLS;
-
-// The plain step on the deviation-collision formats goes through the
-// row-staged kernel (stream_staged.cuh) wherever its requirements hold.
-#ifndef LBCUBE_SHIFTED_STAGED
-#define LBCUBE_SHIFTED_STAGED 1
-#endif
-constexpr bool kShiftedStaged = LBCUBE_SHIFTED_STAGED != 0;
 
 // BGK, TRT and the D2Q9 / D3Q19 MRT collide on the stored deviations; D3Q27
 // MRT and RLBM decode to f and run the reference operator.
 template <class L, int FMT, int CT>
 using ShiftedPolicy =
     std::conditional_t<CT == kBGK || CT == kTRT || (CT == kMRT && L::Q != 27),
-                       DevStorage<FMT, kShiftedCells<FMT>>,
-                       ShiftedStorage<FMT, kShiftedCells<FMT>>>;
+                       DevStorage<FMT>, ShiftedStorage<FMT>>;
 
 template <class L, int FMT, int CT>
 cudaError_t launch_shifted_step(const void* cur, void* nxt, size_t nx, size_t ny, size_t nz,
@@ -52,24 +37,12 @@ cudaError_t launch_shifted_step(const void* cur, void* nxt, size_t nx, size_t ny
   const Span reads[1] = {{cur, bytes}};
   const Span writes[1] = {{nxt, bytes}};
   if (any_overlap(reads, writes)) return cudaErrorInvalidValue;
-  // the public contract for every format: x_extent a multiple of 4, buffers
-  // 8-byte aligned (covers the word shape of both cell counts)
-  if (g.nx % 4 != 0 || (uintptr_t)cur % 8 != 0 || (uintptr_t)nxt % 8 != 0)
-    return cudaErrorInvalidValue;
-  if (!vec_eligible<S>(g, cur, nxt)) return cudaErrorInvalidValue;  // nx % V, word alignment
+  // the public contract for every format: x_extent a multiple of 4, buffers 8-byte aligned
+  if (!codes_eligible(g, cur, nxt)) return cudaErrorInvalidValue;
   const float omega_minus = CT == kTRT ? trt_omega_minus<float>(omega) : 0.0f;
-  if constexpr (kShiftedStaged && S::kBudgeted && S::V == 4 && L::Q <= 19) {
-    if (staged_eligible<L>(g, cur, nxt))
-      return launch_staged_step<L, S, CT>(g, stream, static_cast<const unsigned short*>(cur),
-                                          static_cast<unsigned short*>(nxt), omega, omega_minus,
-                                          typename S::Params{rho0});
-  }
-  const VecGrid vg = make_vec_grid(g, S::V);
-  launch_vec_step<L, S, CT>(vg, vec_grid_dims(vg), vec_block_threads(vg), stream,
-                            static_cast<const unsigned short*>(cur),
-                            static_cast<unsigned short*>(nxt), omega,
-                            omega_minus, typename S::Params{rho0});
-  return cudaGetLastError();
+  return launch_code_step<L, S, CT>(g, stream, static_cast<const unsigned short*>(cur),
+                                    static_cast<unsigned short*>(nxt), omega, omega_minus,
+                                    typename S::Params{rho0}, 0, g.nz);
 }
 
 template <class L, int FMT>
@@ -98,11 +71,11 @@ cudaError_t shifted_by_lattice(int lattice, int collision, const void* cur, void
 // ---- z-slab form -----------------------------------------------------------------
 // One step of planes [z_begin, z_end) of a z-slab of a box on 16-bit storage:
 // populations crossing a face are pulled from halo buffers of codes and the
-// leaving codes stored into send buffers (layout of lbm_slab_face_elems). Where
-// the row-staged kernel applies it steps every plane of the range, its bulk
-// copies reading the halo rows at the faces, so a box stepped as slabs gives
-// the bits of the box stepped whole; otherwise the vectorised kernel steps the
-// interior planes and its SLAB form the face planes.
+// leaving codes stored into send buffers (layout of lbm_slab_face_elems). The
+// whole-box kernel steps the interior planes, which pull and send nothing across
+// a face, and its SLAB form the face planes; every cell does the arithmetic of
+// the whole-box step on the same pairs, so a box stepped as slabs gives the bits
+// of the box stepped whole.
 template <class L, int FMT, int CT>
 cudaError_t launch_shifted_slab_step(const void* cur_v, void* nxt_v, size_t nx, size_t ny,
                                      size_t nz, float omega, float rho0, const void* hl_v,
@@ -130,45 +103,21 @@ cudaError_t launch_shifted_slab_step(const void* cur_v, void* nxt_v, size_t nx, 
   if (any_overlap(reads, writes)) return cudaErrorInvalidValue;
   // the public contract of the 16-bit step (x_extent a multiple of 4, 8-byte
   // aligned buffers), face buffers included
-  if (g.nx % 4 != 0 || !vec_eligible<S>(g, cur, nxt)) return cudaErrorInvalidValue;
+  if (!codes_eligible(g, cur, nxt)) return cudaErrorInvalidValue;
   for (const void* q : {hl_v, hh_v, (const void*)sl, (const void*)sh})
     if ((uintptr_t)q % 8 != 0) return cudaErrorInvalidValue;
   const float omega_minus = CT == kTRT ? trt_omega_minus<float>(omega) : 0.0f;
   const typename S::Params p{rho0};
   const SlabArgs<E> faces{hl, hh, sl, sh, 0};
-  if constexpr (kShiftedStaged && S::kBudgeted && S::V == 4 && L::Q <= 19) {
-    bool faces16 = true;
-    for (const void* q : {hl_v, hh_v, (const void*)sl, (const void*)sh})
-      faces16 = faces16 && (uintptr_t)q % 16 == 0;
-    if (faces16 && staged_eligible<L>(g, cur, nxt))
-      return launch_staged_step<L, S, CT, true>(g, stream, cur, nxt, omega, omega_minus, p,
-                                                (int)z_begin, (int)z_end, faces);
-  }
-  VecGrid vg = make_vec_grid(g, S::V);
-  const size_t ib = std::max<size_t>(z_begin, 1), ie = std::min<size_t>(z_end, nz - 1);
-  if (ib < ie) {
-    vg.z0 = (int)ib;
-    dim3 grid = vec_grid_dims(vg);
-    grid.y = (unsigned)(ie - ib);
-    launch_vec_step<L, S, CT>(vg, grid, vec_block_threads(vg), stream, cur, nxt, omega, omega_minus, p);
-    vg.z0 = 0;
-  }
-  // `count` face planes from z, `step` apart (both faces in one launch where
-  // the range has both)
-  auto face = [&](size_t z, unsigned count, int step) {
-    dim3 grid = vec_grid_dims(vg);
-    grid.y = count;
-    SlabArgs<E> f = faces;
-    f.z_begin = (int)z;
-    f.z_step = step;
-    launch_pdl(fluid_step_vec_kernel<L, S, CT, false, true>, grid, dim3(vec_block_threads(vg)), 0, stream,
-               cur, nxt, vg, omega, omega_minus, p, (double*)nullptr, f);
-  };
-  if (lo_face && hi_face && nz > 1) {
-    face(0, 2, (int)nz - 1);
+  const int ib = (int)std::max<size_t>(z_begin, 1), ie = (int)std::min<size_t>(z_end, nz - 1);
+  if (ib < ie)
+    launch_code_step<L, S, CT>(g, stream, cur, nxt, omega, omega_minus, p, ib, ie - ib);
+  if (lo_face && hi_face && nz > 1) {  // both faces in one launch
+    launch_code_step<L, S, CT>(g, stream, cur, nxt, omega, omega_minus, p, 0, 2, (int)nz - 1, &faces);
   } else {
-    if (lo_face) face(0, 1, 1);
-    if (hi_face && nz > 1) face(nz - 1, 1, 1);
+    if (lo_face) launch_code_step<L, S, CT>(g, stream, cur, nxt, omega, omega_minus, p, 0, 1, 1, &faces);
+    if (hi_face && nz > 1)
+      launch_code_step<L, S, CT>(g, stream, cur, nxt, omega, omega_minus, p, (int)nz - 1, 1, 1, &faces);
   }
   return cudaGetLastError();
 }
@@ -351,14 +300,10 @@ extern "C" int lbm_step_slab_shifted_async(int lattice, int format, int collisio
   return (int)cudaErrorInvalidValue;
 }
 
-extern "C" unsigned int lbm_stage_timeouts(int reset) {
-  unsigned int n = 0;
-  if (cudaMemcpyFromSymbol(&n, g_stage_timeouts, sizeof(n)) != cudaSuccess) return ~0u;
-  if (reset) {
-    const unsigned int zero = 0;
-    if (cudaMemcpyToSymbol(g_stage_timeouts, &zero, sizeof(zero)) != cudaSuccess) return ~0u;
-  }
-  return n;
+// No kernel of the 16-bit step waits for a copy, so none can give up: the
+// count is 0 once the launched work has ended without an error.
+extern "C" unsigned int lbm_stage_timeouts(int) {
+  return cudaStreamSynchronize(cudaStreamLegacy) == cudaSuccess ? 0u : ~0u;
 }
 
 extern "C" int lbm_encode_shifted_async(int lattice, int format, int precision,

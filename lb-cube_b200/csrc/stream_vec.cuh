@@ -13,11 +13,11 @@
 // warp never spans two rows (threads along x are a multiple of 32), so the
 // lane before an active lane always holds the cells just before it.
 //
-// The storage format is a policy:
-//   NativeStorage<Real, V>  FP32/FP64 populations (bit-identical to the one-cell
-//                           kernel: same collision code, only the memory access differs)
-//   ShiftedStorage<fmt, V>  16-bit shifted populations decoded to FP32 f
-//   DevStorage<fmt, V>      16-bit shifted populations collided as deviations
+// The storage format is a policy, NativeStorage<Real, V>: FP32/FP64 populations
+// (bit-identical to the one-cell kernel: same collision code, only the memory
+// access differs). The policies of the 16-bit step (stream_codes.cuh) follow it:
+//   ShiftedStorage<fmt>  16-bit shifted populations decoded to FP32 f
+//   DevStorage<fmt>      16-bit shifted populations collided as deviations
 #pragma once
 
 #include <cuda_bf16.h>
@@ -48,7 +48,6 @@ struct NativeStorage {
   using elem = Real;
   using compute = Real;
   static constexpr int V = VEC;
-  static constexpr bool kBudgeted = false;
   struct Params {};
   template <class L, int i>
   __device__ __forceinline__ static compute decode(elem v, const Params&) { return v; }
@@ -82,95 +81,58 @@ struct NativeStorage {
 // puts every direction on the same scale, and S places that range where the
 // format resolves it best. This policy decodes to f and runs the reference
 // collision (MRT, RLBM, conversions); DevStorage below collides on v directly.
-template <int FMT, int VEC = 4>
+template <int FMT>
 struct ShiftedStorage {
   using elem = unsigned short;
-  using compute = float;
-  static constexpr int V = VEC;  // cells per thread, decoded to FP32 in registers
-  static constexpr bool kBudgeted = false;
+  static constexpr bool kDecoded = true;
   struct Params {
     float rho0;
   };
   template <class L, int i>
-  __device__ __forceinline__ static compute decode(elem h, const Params& p) {
+  __device__ __forceinline__ static float decode(elem h, const Params& p) {
     constexpr double wd = L::w[i];
     return float(wd) * fmaf(Codec<FMT>::decode(h), 1.0f / Codec<FMT>::S, p.rho0);
   }
   template <class L, int i>
-  __device__ __forceinline__ static elem encode(compute f, const Params& p) {
+  __device__ __forceinline__ static elem encode(float f, const Params& p) {
     constexpr double wd = L::w[i];
     return Codec<FMT>::encode((f * float(1.0 / wd) - p.rho0) * Codec<FMT>::S);
   }
   template <class L, int i>
-  __device__ __forceinline__ static void decode_word(const RowWord<elem, V>& w, compute (&out)[V],
-                                                     const Params& p) {
-#pragma unroll
-    for (int j = 0; j < V; ++j) out[j] = decode<L, i>(w.v[j], p);
+  __device__ __forceinline__ static float2 decode_pair(unsigned int w, const Params& p) {
+    return make_float2(decode<L, i>((elem)w, p), decode<L, i>((elem)(w >> 16), p));
   }
   template <class L, int i>
-  __device__ __forceinline__ static RowWord<elem, V> encode_word(const compute (&in)[V],
-                                                                const Params& p) {
-    RowWord<elem, V> w;
-#pragma unroll
-    for (int j = 0; j < V; ++j) w.v[j] = encode<L, i>(in[j], p);
-    return w;
+  __device__ __forceinline__ static unsigned int encode_pair(float a, float b, const Params& p) {
+    return __byte_perm(encode<L, i>(a, p), encode<L, i>(b, p), 0x5410);
   }
   template <class L, int CT>
-  __device__ __forceinline__ static void collide_cell(compute (&f)[L::Q], compute omega,
-                                                      compute omega_minus, const Params&) {
-    collide<L, compute, CT>(f, omega, omega_minus);
+  __device__ __forceinline__ static void collide_cell(float (&f)[L::Q], float omega, float omega_minus,
+                                                      const Params&) {
+    collide<L, float, CT>(f, omega, omega_minus);
   }
 };
 
-// 16-bit storage whose collision runs on the stored deviations (BGK, TRT).
-template <int FMT, int VEC = 4>
+// 16-bit storage whose collision runs on the stored deviations (BGK, TRT, and
+// the D2Q9 / D3Q19 MRT).
+template <int FMT>
 struct DevStorage {
-  static_assert(VEC % 2 == 0, "codes are converted in pairs");
   using elem = unsigned short;
-  using compute = float;
-  static constexpr int V = VEC;
-  static constexpr bool kBudgeted = true;
+  static constexpr bool kDecoded = false;
   struct Params {
     float rho0;
   };
   template <class L, int i>
-  __device__ __forceinline__ static compute decode(elem h, const Params&) {
-    return Codec<FMT>::decode(h);
+  __device__ __forceinline__ static float2 decode_pair(unsigned int w, const Params&) {
+    return Codec<FMT>::decode2(w);
   }
   template <class L, int i>
-  __device__ __forceinline__ static elem encode(compute v, const Params&) {
-    return Codec<FMT>::encode(v);
-  }
-  // V is even: the word holds V/2 32-bit pairs, converted pairwise.
-  template <class L, int i>
-  __device__ __forceinline__ static void decode_word(const RowWord<elem, V>& w, compute (&out)[V],
-                                                     const Params&) {
-    unsigned int u[V / 2];
-    memcpy(u, &w, sizeof(u));
-#pragma unroll
-    for (int k = 0; k < V / 2; ++k) {
-      const float2 d = Codec<FMT>::decode2(u[k]);
-      out[2 * k] = d.x;
-      out[2 * k + 1] = d.y;
-    }
-  }
-  template <class L, int i>
-  __device__ __forceinline__ static RowWord<elem, V> encode_word(const compute (&in)[V],
-                                                                const Params&) {
-    unsigned int u[V / 2];
-#pragma unroll
-    for (int k = 0; k < V / 2; ++k) u[k] = Codec<FMT>::encode2(in[2 * k], in[2 * k + 1]);
-    RowWord<elem, V> w;
-    memcpy(&w, u, sizeof(u));
-    return w;
-  }
-  __device__ __forceinline__ static float2 decode_pair(unsigned int w) { return Codec<FMT>::decode2(w); }
-  __device__ __forceinline__ static unsigned int encode_pair(float a, float b) {
+  __device__ __forceinline__ static unsigned int encode_pair(float a, float b, const Params&) {
     return Codec<FMT>::encode2(a, b);
   }
   template <class L, int CT>
-  __device__ __forceinline__ static void collide_cell(compute (&v)[L::Q], compute omega,
-                                                      compute omega_minus, const Params& p) {
+  __device__ __forceinline__ static void collide_cell(float (&v)[L::Q], float omega, float omega_minus,
+                                                      const Params& p) {
     static_assert(CT == kBGK || CT == kTRT || (CT == kMRT && L::Q != 27),
                   "deviation-space collision is BGK, TRT, or D2Q9 / D3Q19 MRT");
     if constexpr (CT == kMRT) collide_dev_mrt<L, FMT>(v, omega, p.rho0);
@@ -398,45 +360,20 @@ __global__ void __launch_bounds__(kThreads)
   fluid_step_vec_body<L, S, CT, DIAG, SLAB>(cur, nxt, vg, omega, omega_minus, p, partials, slab);
 }
 
-// The plain step on 16-bit storage with a register budget: at least
-// kShiftedMinBlocks blocks of kThreads per SM. Four cells of 19 populations per
-// thread leave the compiler free to interleave the cells' collisions up to
-// 128 registers (4 blocks per SM), which an issue-bound kernel pays for in
-// latency it cannot hide.
-#ifndef LBCUBE_SHIFTED_MIN_BLOCKS
-#define LBCUBE_SHIFTED_MIN_BLOCKS 5
-#endif
-constexpr int kShiftedMinBlocks = LBCUBE_SHIFTED_MIN_BLOCKS;
-
-template <class L, class S, int CT>
-__global__ void __launch_bounds__(kThreads, kShiftedMinBlocks)
-    fluid_step_vec16_kernel(const typename S::elem* __restrict__ cur,
-                            typename S::elem* __restrict__ nxt, VecGrid vg,
-                            typename S::compute omega, typename S::compute omega_minus,
-                            typename S::Params p) {
-  fluid_step_vec_body<L, S, CT, false, false>(cur, nxt, vg, omega, omega_minus, p, nullptr, {});
-}
-
 // Launches the plain vectorised step. (Register budgets, i.e. launch bounds
 // with a minimum block count, were timed at 4..8 blocks per SM for every
-// lattice, precision and operator of the native storage; where they won, for
-// FP32 D3Q19 MRT and RLBM, the one-cell kernel (step_cell.cuh) won by more and
-// now runs those. An explicit count of 1 is not the compiler's default: it
-// lets the allocation grow, e.g. 64 -> 94 registers for the FP32 D3Q19 TRT
-// step.) 16-bit storage colliding on the deviations runs the budgeted kernel
-// above for D2Q9 and D3Q19 (D3Q27 and the decoded RLBM spill under it).
+// lattice, precision and operator; where they won, for FP32 D3Q19 MRT and RLBM,
+// the one-cell kernel (step_cell.cuh) won by more and now runs those. An
+// explicit count of 1 is not the compiler's default: it lets the allocation
+// grow, e.g. 64 -> 94 registers for the FP32 D3Q19 TRT step.)
 template <class L, class S, int CT>
 inline void launch_vec_step(const VecGrid& vg, dim3 grid, unsigned threads, cudaStream_t stream,
                             const typename S::elem* cur, typename S::elem* nxt,
                             typename S::compute omega, typename S::compute omega_minus,
                             const typename S::Params& p) {
-  // programmatic dependent launches (pdl_enter opens the body)
-  if constexpr (S::kBudgeted && L::Q <= 19)
-    launch_pdl(fluid_step_vec16_kernel<L, S, CT>, grid, dim3(threads), 0, stream, cur, nxt, vg, omega,
-               omega_minus, p);
-  else
-    launch_pdl(fluid_step_vec_kernel<L, S, CT, false, false>, grid, dim3(threads), 0, stream, cur, nxt,
-               vg, omega, omega_minus, p, (double*)nullptr, SlabArgs<typename S::elem>{});
+  // a programmatic dependent launch (pdl_enter opens the body)
+  launch_pdl(fluid_step_vec_kernel<L, S, CT, false, false>, grid, dim3(threads), 0, stream, cur, nxt, vg,
+             omega, omega_minus, p, (double*)nullptr, SlabArgs<typename S::elem>{});
 }
 
 template <class S>
