@@ -10,6 +10,8 @@
 // Halves the bytes of the coupled step (D3Q19 + 2 D3Q7: 132 B per cell
 // instead of 264). Statistics, when requested, are those of the FP32 values
 // the step encodes.
+#include <initializer_list>
+
 #include "adr_shifted.cuh"
 #include "cells.cuh"
 #include "collide.cuh"
@@ -17,6 +19,7 @@
 #include "common.cuh"
 #include "reduce.cuh"
 #include "slab_faces.cuh"
+#include "stream_codes.cuh"
 #include "stream_vec.cuh"
 #include "../../include/lbcube_b200.h"
 
@@ -137,6 +140,151 @@ __global__ void __launch_bounds__(kThreads)
   if constexpr (STATS) block_sum_to<kStatSums>(sums, partials + block_linear() * kStatSums);
 }
 
+// The whole-box step with four x-adjacent cells per thread (stream_codes.cuh):
+// one 8-byte word of codes per population instead of four 2-byte accesses. Each
+// cell's arithmetic is that of fluid_reaction_shifted_kernel, so are the codes.
+// The fluid goes first (its 19 words are dead before the scalars' 14 arrive),
+// leaving only the four velocities. FP16 TRT 192^3: 252.8 -> 173.0 us per step
+// (5.4 TB/s), 262.7 -> 178.4 us with the velocity stored; the 12-step gradient at
+// five resident blocks 10.39 ms, at four 10.50, at six (spills) 10.80.
+// STATS: the block's sums go to the first of the partials of the cells it
+// covers (kCodeCells one-cell blocks), zeros to the others, so the second pass
+// reads the same number of partials whichever kernel ran.
+constexpr int kCoupledCodeBlocks = 5;
+template <class FL, int FMT, int CT, bool STATS, bool UOUT>
+__global__ void __launch_bounds__(kThreads, kCoupledCodeBlocks)
+    fluid_reaction_codes_kernel(const unsigned short* __restrict__ cur_f, unsigned short* __restrict__ nxt_f,
+                                const unsigned short* __restrict__ cur_a, unsigned short* __restrict__ nxt_a,
+                                const unsigned short* __restrict__ cur_b, unsigned short* __restrict__ nxt_b,
+                                CodeGrid g, float omega, float omega_minus, float omega_c, float k, float rho0,
+                                float c0, double* __restrict__ partials, int tiles, float* __restrict__ u_out) {
+  using SL = typename ScalarOf<FL>::type;
+  using SS = ShiftedStorage<FMT>;
+  pdl_enter();
+  int x0, y, z;
+  const bool active = word_of(g, x0, y, z);
+  double sums[kStatSums] = {0.0, 0.0, 0.0, 0.0, 0.0};
+  if (active) {
+    const size_t plane = (size_t)g.plane;
+    const int cell = (z * g.ny + y) * g.nx + x0;
+    float u[kCodeCells][FL::D];
+    {
+      unsigned int raw[FL::Q][2];
+      gather_words<FL>(cur_f, g, x0, y, z, raw);
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        float v[2][FL::Q];
+        static_for<FL::Q>([&](auto I) {
+          const float2 d = Codec<FMT>::decode2(raw[LB_I(I)][h]);
+          v[0][LB_I(I)] = d.x;
+          v[1][LB_I(I)] = d.y;
+        });
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          if constexpr (CT == kMRT) collide_dev_mrt<FL, FMT>(v[j], omega, rho0);
+          else collide_dev<FL, CT, FMT>(v[j], omega, omega_minus, rho0);
+          dev_velocity<FL, FMT>(v[j], rho0, u[2 * h + j]);
+        }
+        static_for<FL::Q>([&](auto I) {
+          raw[LB_I(I)][h] =
+              __byte_perm(Codec<FMT>::encode(v[0][LB_I(I)]), Codec<FMT>::encode(v[1][LB_I(I)]), 0x5410);
+        });
+      }
+      static_for<FL::Q>([&](auto I) {
+        *reinterpret_cast<uint2*>(nxt_f + plane * LB_I(I) + cell) = make_uint2(raw[LB_I(I)][0], raw[LB_I(I)][1]);
+      });
+    }
+    if constexpr (UOUT)
+      static_for<FL::D>([&](auto D) {
+        *reinterpret_cast<float4*>(u_out + plane * LB_I(D) + cell) =
+            make_float4(u[0][LB_I(D)], u[1][LB_I(D)], u[2][LB_I(D)], u[3][LB_I(D)]);
+      });
+    unsigned int ra[SL::Q][2], rb[SL::Q][2];
+    gather_words<SL>(cur_a, g, x0, y, z, ra);
+    gather_words<SL>(cur_b, g, x0, y, z, rb);
+    const typename SS::Params sp{c0};
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      float a[2][SL::Q], b[2][SL::Q];
+      static_for<SL::Q>([&](auto I) {
+        constexpr int i = LB_I(I);
+        const float2 da = SS::template decode_pair<SL, i>(ra[i][h], sp);
+        const float2 db = SS::template decode_pair<SL, i>(rb[i][h], sp);
+        a[0][i] = da.x;
+        a[1][i] = da.y;
+        b[0][i] = db.x;
+        b[1][i] = db.y;
+      });
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        react_pair<SL>(a[j], b[j], u[2 * h + j], omega_c, k);
+        if constexpr (STATS) {
+          const double sa = (double)concentration<SL>(a[j]), sb = (double)concentration<SL>(b[j]);
+          sums[0] += sa;
+          sums[1] += sb;
+          sums[2] += sa * sa;
+          sums[3] += sb * sb;
+          sums[4] += sa * sb;
+        }
+      }
+      static_for<SL::Q>([&](auto I) {
+        constexpr int i = LB_I(I);
+        ra[i][h] = SS::template encode_pair<SL, i>(a[0][i], a[1][i], sp);
+        rb[i][h] = SS::template encode_pair<SL, i>(b[0][i], b[1][i], sp);
+      });
+    }
+    static_for<SL::Q>([&](auto I) {
+      constexpr int i = LB_I(I);
+      *reinterpret_cast<uint2*>(nxt_a + plane * i + cell) = make_uint2(ra[i][0], ra[i][1]);
+      *reinterpret_cast<uint2*>(nxt_b + plane * i + cell) = make_uint2(rb[i][0], rb[i][1]);
+    });
+  }
+  if constexpr (STATS) {
+    const int first = (int)blockIdx.x * kCodeCells;
+    double* const out = partials + ((long long)z * tiles + first) * kStatSums;
+    block_sum_to<kStatSums>(sums, out);
+    const int rest = (min(kCodeCells, tiles - first) - 1) * kStatSums;
+    if ((int)threadIdx.x < rest) out[kStatSums + threadIdx.x] = 0.0;
+  }
+}
+
+// Whether the four-cell kernel steps a range of planes: whole words per row,
+// word-aligned buffers, and a 16-byte aligned velocity output. D3Q27 keeps the
+// one-cell kernel (its 27 words alone fill the register budget).
+template <class FL>
+inline bool coupled_codes_eligible(const Grid& g, std::initializer_list<const void*> codes, const float* u_out) {
+  if (FL::Q > 19 || g.nx % kCodeCells != 0 || (uintptr_t)u_out % 16 != 0) return false;
+  for (const void* p : codes)
+    if ((uintptr_t)p % 8 != 0) return false;
+  return true;
+}
+
+// Planes [z0, z0 + planes) without the faces of a slab, by whichever kernel applies.
+template <class FL, int FMT, int CT, bool STATS, bool UOUT>
+cudaError_t launch_coupled_planes(const unsigned short* cf, unsigned short* nf, const unsigned short* ca,
+                                  unsigned short* na, const unsigned short* cb, unsigned short* nb,
+                                  float* u_out, double* partials, const Grid& g, int z0, int planes,
+                                  float omega, float om, float omega_c, float k, float rho0, float c0,
+                                  cudaStream_t s) {
+  // programmatic dependent launches (the kernels open with pdl_enter)
+  if constexpr (FL::Q <= 19) {
+    if (coupled_codes_eligible<FL>(g, {cf, nf, ca, na, cb, nb}, u_out)) {
+      const CodeGrid cg = make_code_grid(g, z0);
+      const unsigned words = (unsigned)(cg.words * g.ny);
+      return launch_pdl(fluid_reaction_codes_kernel<FL, FMT, CT, STATS, UOUT>,
+                        dim3((words + kThreads - 1) / kThreads, (unsigned)planes), dim3(kThreads), 0, s, cf, nf,
+                        ca, na, cb, nb, cg, omega, om, omega_c, k, rho0, c0, partials, g.tiles, u_out);
+    }
+  }
+  Grid gr = g;
+  gr.z0 = z0;
+  dim3 grid = grid_dims(gr);
+  grid.y = (unsigned)planes;
+  return launch_pdl(fluid_reaction_shifted_kernel<FL, FMT, CT, STATS, UOUT, false>, grid, dim3(block_dims(gr)),
+                    0, s, cf, nf, ca, na, cb, nb, gr, omega, om, omega_c, k, rho0, c0, partials, u_out,
+                    CodeFaces{});
+}
+
 template <class FL, int FMT, int CT>
 cudaError_t launch_shifted_coupled(const unsigned short* cf, unsigned short* nf,
                                    const unsigned short* ca, unsigned short* na,
@@ -144,11 +292,9 @@ cudaError_t launch_shifted_coupled(const unsigned short* cf, unsigned short* nf,
                                    double* partials, const Grid& g, float omega, float omega_c,
                                    float k, float rho0, float c0, cudaStream_t s) {
   const float om = CT == kTRT ? trt_omega_minus<float>(omega) : 0.0f;
-  // programmatic dependent launches (the kernel opens with pdl_enter)
-#define LBCUBE_SC(ST, UO)                                                                          \
-  return launch_pdl(fluid_reaction_shifted_kernel<FL, FMT, CT, ST, UO, false>, grid_dims(g),      \
-                    dim3(block_dims(g)), 0, s, cf, nf, ca, na, cb, nb, g, omega, om, omega_c, k,  \
-                    rho0, c0, partials, u_out, CodeFaces{})
+#define LBCUBE_SC(ST, UO)                                                                            \
+  return launch_coupled_planes<FL, FMT, CT, ST, UO>(cf, nf, ca, na, cb, nb, u_out, partials, g, 0, g.nz, \
+                                                    omega, om, omega_c, k, rho0, c0, s)
   if (partials != nullptr && u_out != nullptr) LBCUBE_SC(true, true);
   if (partials != nullptr) LBCUBE_SC(true, false);
   if (u_out != nullptr) LBCUBE_SC(false, true);
@@ -197,25 +343,26 @@ cudaError_t fluid_reaction_shifted_slab(int collision, const unsigned short* cur
   auto launch = [&](auto ct) -> cudaError_t {
     constexpr int CT = decltype(ct)::value;
     const float om = CT == kTRT ? trt_omega_minus<float>(omega) : 0.0f;
-    auto range = [&](int z0, int planes, int zs, auto slab) {
-      constexpr bool SLAB = decltype(slab)::value;
-      Grid gr = g;
-      gr.z0 = z0;
-      gr.zs = zs;
-      dim3 grid = grid_dims(gr);
-      grid.y = (unsigned)planes;
-      const dim3 block(block_dims(gr));
-      double* const none = nullptr;
+    double* const none = nullptr;
+    if (g.nz >= 3) {
       if (u_out != nullptr)
-        launch_pdl(fluid_reaction_shifted_kernel<FL, FMT, CT, false, true, SLAB>, grid, block, 0, s, cur_f,
-                   nxt_f, cur_a, nxt_a, cur_b, nxt_b, gr, omega, om, omega_c, k, rho0, c0, none, u_out, faces);
+        launch_coupled_planes<FL, FMT, CT, false, true>(cur_f, nxt_f, cur_a, nxt_a, cur_b, nxt_b, u_out, none, g,
+                                                        1, g.nz - 2, omega, om, omega_c, k, rho0, c0, s);
       else
-        launch_pdl(fluid_reaction_shifted_kernel<FL, FMT, CT, false, false, SLAB>, grid, block, 0, s, cur_f,
-                   nxt_f, cur_a, nxt_a, cur_b, nxt_b, gr, omega, om, omega_c, k, rho0, c0, none,
-                   (float*)nullptr, faces);
-    };
-    if (g.nz >= 3) range(1, g.nz - 2, 1, std::false_type{});
-    range(0, g.nz >= 2 ? 2 : 1, g.nz - 1, std::true_type{});  // both face planes in one launch
+        launch_coupled_planes<FL, FMT, CT, false, false>(cur_f, nxt_f, cur_a, nxt_a, cur_b, nxt_b, u_out, none,
+                                                         g, 1, g.nz - 2, omega, om, omega_c, k, rho0, c0, s);
+    }
+    Grid gr = g;  // both face planes in one launch
+    gr.zs = g.nz - 1;
+    dim3 grid = grid_dims(gr);
+    grid.y = g.nz >= 2 ? 2 : 1;
+    const dim3 block(block_dims(gr));
+    if (u_out != nullptr)
+      launch_pdl(fluid_reaction_shifted_kernel<FL, FMT, CT, false, true, true>, grid, block, 0, s, cur_f, nxt_f,
+                 cur_a, nxt_a, cur_b, nxt_b, gr, omega, om, omega_c, k, rho0, c0, none, u_out, faces);
+    else
+      launch_pdl(fluid_reaction_shifted_kernel<FL, FMT, CT, false, false, true>, grid, block, 0, s, cur_f, nxt_f,
+                 cur_a, nxt_a, cur_b, nxt_b, gr, omega, om, omega_c, k, rho0, c0, none, (float*)nullptr, faces);
     return cudaGetLastError();
   };
   switch (collision) {
