@@ -18,6 +18,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
@@ -104,6 +105,28 @@ def build_drivers(force: bool = False) -> list:
     return out
 
 
+CALL = os.path.join(HERE, "_lbcall.so")
+
+
+def build_call(force: bool = False):
+    """The native call path of lbcube.py (csrc/pycall.c), an extension module of
+    this Python. Without its headers nothing is built and lbcube.py calls
+    through ctypes."""
+    inc = sysconfig.get_paths()["include"]
+    src = os.path.join(CSRC, "pycall.c")
+    if not os.path.exists(os.path.join(inc, "Python.h")):
+        return None
+    if force or _stale(CALL, [src]):
+        cc = os.environ.get("CC", shutil.which("gcc") or "gcc")
+        cmd = [cc, "-O2", "-fPIC", "-shared", "-Wall", "-Wextra", "-Wno-unused-parameter", f"-I{inc}", src, "-o",
+               CALL + ".tmp"]
+        res = subprocess.run(cmd, capture_output=True, text=True)
+        if res.returncode != 0:
+            raise RuntimeError(f"call path build failed:\n{' '.join(cmd)}\n{res.stdout}\n{res.stderr}")
+        os.replace(CALL + ".tmp", CALL)
+    return CALL
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
     """Compile (if stale) and link the engine library; returns its path."""
     os.makedirs(BUILD, exist_ok=True)
@@ -127,6 +150,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
             raise RuntimeError(f"link failed:\n{' '.join(cmd)}\n{res.stdout}\n{res.stderr}")
         os.replace(tmp, LIB)
     build_drivers(force)
+    build_call(force)
     return LIB
 
 

@@ -41,6 +41,9 @@ STATS_FIELDS = ("mean_A", "mean_B", "var_A", "var_B", "covariance", "segregation
                 "true_reaction_rate", "mixed_reaction_rate")
 
 _lib = None
+_call = None  # the native call path of the step launchers (csrc/pycall.c), or None: ctypes only
+CALL_PATH = os.path.join(HERE, "_lbcall.so")
+_BLOCK = (16, 8, 1)  # the reference's default block
 
 
 class LbmCudaError(RuntimeError):
@@ -55,15 +58,39 @@ def library_path() -> str:
 
 def load() -> C.CDLL:
     """The engine library, loaded once. Raises if it has not been built."""
-    global _lib
+    global _lib, _call
     if _lib is None:
         if not os.path.exists(LIB_PATH):
             raise RuntimeError(
                 f"engine library {LIB_PATH} is missing: build it with "
                 "`python lb-cube_b200/build.py` (there is no CPU fallback)")
-        _lib = C.CDLL(LIB_PATH)
-        _declare(_lib)
+        lib = C.CDLL(LIB_PATH)
+        _declare(lib)
+        _call = _load_call(lib)
+        _lib = lib
     return _lib
+
+
+def _load_call(lib):
+    """The extension module that calls the step launchers without ctypes'
+    argument conversion, bound to this library; None where it was not built.
+    Its functions return None for arguments other than plain names, ints,
+    floats and buffers, which then take the ctypes path."""
+    if not os.path.exists(CALL_PATH):
+        return None
+    from importlib.machinery import ExtensionFileLoader
+    from importlib.util import module_from_spec, spec_from_file_location
+
+    try:
+        spec = spec_from_file_location("_lbcall", CALL_PATH, loader=ExtensionFileLoader("_lbcall", CALL_PATH))
+        mod = module_from_spec(spec)
+        spec.loader.exec_module(mod)
+    except ImportError:  # built for another Python
+        return None
+    mod.setup(*(C.cast(getattr(lib, n), C.c_void_p).value for n in (
+        "lbm_step_async", "lbm_step_shifted_async", "lbm_scalar_step_async", "lbm_reaction_ab_async",
+        "lbm_fluid_reaction_ab_async")))
+    return mod
 
 
 _sz, _vp, _u = C.c_size_t, C.c_void_p, C.c_uint
@@ -208,15 +235,20 @@ def check(code: int, what: str = "launch") -> None:
 # Reference-named launchers (return the cudaError_t code, like the reference)
 # --------------------------------------------------------------------------
 def launch_step_gpu(lattice, real, collision, current_populations, next_populations, x_extent,
-                    y_extent, z_extent, omega, block=(16, 8, 1)) -> int:
+                    y_extent, z_extent, omega, block=_BLOCK) -> int:
     """lbm::launch_step_gpu<Lattice, Real, CT> (include/lattice_cuda.cuh:179-190)."""
+    if _call is not None and block is _BLOCK:  # the same launch on the default stream
+        rc = _call.step(lattice, real, collision, current_populations, next_populations, x_extent, y_extent,
+                        z_extent, omega, None)
+        if rc is not None:
+            return rc
     fn = getattr(load(), f"lbm_launch_step_gpu_{lattice.lower()}_{real_name(real)}_{collision.lower()}")
     return fn(_ptr(current_populations), _ptr(next_populations), x_extent, y_extent, z_extent,
               omega, *block)
 
 
 def launch_step_gpu_mem(lattice, real, collision, mem_extents, current_populations,
-                        next_populations, omega, block=(16, 8, 1)) -> int:
+                        next_populations, omega, block=_BLOCK) -> int:
     """The LatticeMemory overload (include/lattice_cuda.cuh:310-319): extents from a memory object."""
     nx, ny, nz = mem_extents
     return launch_step_gpu(lattice, real, collision, current_populations, next_populations, nx, ny,
@@ -225,8 +257,13 @@ def launch_step_gpu_mem(lattice, real, collision, mem_extents, current_populatio
 
 def launch_scalar_step_gpu(fluid_lattice, real, current_scalar, next_scalar, current_fluid,
                            x_extent, y_extent, z_extent, omega_c, source_term=0.0,
-                           block=(16, 8, 1)) -> int:
+                           block=_BLOCK) -> int:
     """lbm::launch_scalar_step_gpu<FL, SL, Real> (include/lattice_cuda.cuh:209-222)."""
+    if _call is not None and block is _BLOCK:
+        rc = _call.scalar_step(fluid_lattice, real, current_scalar, next_scalar, current_fluid, x_extent, y_extent,
+                               z_extent, omega_c, source_term, None)
+        if rc is not None:
+            return rc
     sl = SCALAR_OF[fluid_lattice].lower()
     fn = getattr(load(), f"lbm_launch_scalar_step_gpu_{fluid_lattice.lower()}_{sl}_{real_name(real)}")
     return fn(_ptr(current_scalar), _ptr(next_scalar), _ptr(current_fluid), x_extent, y_extent,
@@ -235,7 +272,7 @@ def launch_scalar_step_gpu(fluid_lattice, real, current_scalar, next_scalar, cur
 
 def launch_scalar_step_gpu_mem(fluid_lattice, real, scalar_extents, fluid_extents, current_scalar,
                                next_scalar, current_fluid, omega_c, source_term=0.0,
-                               block=(16, 8, 1)) -> int:
+                               block=_BLOCK) -> int:
     """The LatticeMemory overload (include/lattice_cuda.cuh:243-255, src/lattice_cuda.cu:716-747):
     mismatched scalar/fluid extents return cudaErrorInvalidValue."""
     if tuple(scalar_extents) != tuple(fluid_extents):
@@ -247,8 +284,13 @@ def launch_scalar_step_gpu_mem(fluid_lattice, real, scalar_extents, fluid_extent
 
 def launch_reaction_AB_gpu(fluid_lattice, real, current_a, next_a, current_b, next_b,
                            current_fluid, x_extent, y_extent, z_extent, omega_c, k_react,
-                           block=(16, 8, 1)) -> int:
+                           block=_BLOCK) -> int:
     """lbm::launch_reaction_AB_gpu<FL, SL, Real> (include/lattice_cuda.cuh:276-291)."""
+    if _call is not None and block is _BLOCK:
+        rc = _call.reaction_ab(fluid_lattice, real, current_a, next_a, current_b, next_b, current_fluid, x_extent,
+                               y_extent, z_extent, omega_c, k_react, None)
+        if rc is not None:
+            return rc
     sl = SCALAR_OF[fluid_lattice].lower()
     fn = getattr(load(), f"lbm_launch_reaction_ab_gpu_{fluid_lattice.lower()}_{sl}_{real_name(real)}")
     return fn(_ptr(current_a), _ptr(next_a), _ptr(current_b), _ptr(next_b), _ptr(current_fluid),
@@ -259,12 +301,20 @@ def launch_reaction_AB_gpu(fluid_lattice, real, current_a, next_a, current_b, ne
 # Stream-ordered extensions
 # --------------------------------------------------------------------------
 def step_async(lattice, real, collision, cur, nxt, nx, ny, nz, omega, stream=None) -> int:
+    if _call is not None:
+        rc = _call.step(lattice, real, collision, cur, nxt, nx, ny, nz, omega, stream)
+        if rc is not None:
+            return rc
     return load().lbm_step_async(LATTICES[lattice], REALS[real_name(real)], COLLISIONS[collision],
                                  _ptr(cur), _ptr(nxt), nx, ny, nz, float(omega), _stream(stream))
 
 
 def scalar_step_async(fluid_lattice, real, cur_s, nxt_s, cur_f, nx, ny, nz, omega_c, source=0.0,
                       stream=None) -> int:
+    if _call is not None:
+        rc = _call.scalar_step(fluid_lattice, real, cur_s, nxt_s, cur_f, nx, ny, nz, omega_c, source, stream)
+        if rc is not None:
+            return rc
     return load().lbm_scalar_step_async(LATTICES[fluid_lattice], REALS[real_name(real)], _ptr(cur_s),
                                         _ptr(nxt_s), _ptr(cur_f), nx, ny, nz, float(omega_c),
                                         float(source), _stream(stream))
@@ -272,6 +322,11 @@ def scalar_step_async(fluid_lattice, real, cur_s, nxt_s, cur_f, nx, ny, nz, omeg
 
 def reaction_ab_async(fluid_lattice, real, cur_a, nxt_a, cur_b, nxt_b, cur_f, nx, ny, nz, omega_c,
                       k_react, stream=None) -> int:
+    if _call is not None:
+        rc = _call.reaction_ab(fluid_lattice, real, cur_a, nxt_a, cur_b, nxt_b, cur_f, nx, ny, nz, omega_c, k_react,
+                               stream)
+        if rc is not None:
+            return rc
     return load().lbm_reaction_ab_async(LATTICES[fluid_lattice], REALS[real_name(real)], _ptr(cur_a),
                                         _ptr(nxt_a), _ptr(cur_b), _ptr(nxt_b), _ptr(cur_f), nx, ny,
                                         nz, float(omega_c), float(k_react), _stream(stream))
@@ -284,6 +339,11 @@ def stats_partials_bytes(fluid_lattice, nx, ny, nz) -> int:
 def fluid_reaction_ab_async(fluid_lattice, real, collision, cur_f, nxt_f, cur_a, nxt_a, cur_b, nxt_b,
                             nx, ny, nz, omega, omega_c, k_react, partials=None, partials_bytes=0,
                             stream=None) -> int:
+    if _call is not None:
+        rc = _call.fluid_reaction_ab(fluid_lattice, real, collision, cur_f, nxt_f, cur_a, nxt_a, cur_b, nxt_b, nx, ny,
+                                     nz, omega, omega_c, k_react, partials, partials_bytes, stream)
+        if rc is not None:
+            return rc
     return load().lbm_fluid_reaction_ab_async(
         LATTICES[fluid_lattice], REALS[real_name(real)], COLLISIONS[collision], _ptr(cur_f),
         _ptr(nxt_f), _ptr(cur_a), _ptr(nxt_a), _ptr(cur_b), _ptr(nxt_b), nx, ny, nz, float(omega),
@@ -332,6 +392,10 @@ def init_equilibrium_async(lattice, real, rho, u, populations, nx, ny, nz, strea
 def step_shifted_async(lattice, fmt, collision, cur, nxt, nx, ny, nz, omega, rho0=1.0,
                        stream=None) -> int:
     """One collide-stream step on shifted 16-bit populations (fmt in FORMATS)."""
+    if _call is not None:
+        rc = _call.step_shifted(lattice, fmt, collision, cur, nxt, nx, ny, nz, omega, rho0, stream)
+        if rc is not None:
+            return rc
     return load().lbm_step_shifted_async(LATTICES[lattice], FORMATS[fmt], COLLISIONS[collision],
                                          _ptr(cur), _ptr(nxt), nx, ny, nz, float(omega),
                                          float(rho0), _stream(stream))
