@@ -42,11 +42,11 @@
 #include "adr.cuh"
 #include "adr_shifted.cuh"
 #include "cells.cuh"
+#include "codes.cuh"
 #include "collide.cuh"
 #include "common.cuh"
 #include "reduce.cuh"
 #include "slab_faces.cuh"
-#include "stream_vec.cuh"
 #include "../../include/lbcube_b200.h"
 
 namespace lbcube {

@@ -20,7 +20,6 @@
 #include "reduce.cuh"
 #include "slab_faces.cuh"
 #include "stream_codes.cuh"
-#include "stream_vec.cuh"
 #include "../../include/lbcube_b200.h"
 
 namespace lbcube {

@@ -6,6 +6,7 @@
 #include <climits>
 #include <cstddef>
 #include <cstdint>
+#include <type_traits>
 #include <utility>
 
 #include "lattices.cuh"
@@ -78,6 +79,36 @@ __device__ __forceinline__ long long block_linear() {
   return (long long)blockIdx.y * gridDim.x + blockIdx.x;
 }
 
+// The load of a pulled population, through the read-only path; FIRST: with the
+// L2 policy that evicts its line first.
+template <bool FIRST>
+struct PullLoad {
+  unsigned long long policy = 0;
+  __device__ __forceinline__ PullLoad() {
+    if constexpr (FIRST) asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
+  }
+  template <class T>
+  __device__ __forceinline__ T operator()(const T* p) const {
+    if constexpr (!FIRST) {
+      return __ldg(p);
+    } else if constexpr (std::is_same_v<T, float>) {
+      float v;
+      asm volatile("ld.global.nc.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(v) : "l"(p), "l"(policy));
+      return v;
+    } else if constexpr (std::is_same_v<T, float2>) {
+      float2 v;
+      asm volatile("ld.global.nc.L2::cache_hint.v2.f32 {%0, %1}, [%2], %3;"
+                   : "=f"(v.x), "=f"(v.y) : "l"(p), "l"(policy));
+      return v;
+    } else {
+      static_assert(std::is_same_v<T, double>, "float, float2 or double");
+      double v;
+      asm volatile("ld.global.nc.L2::cache_hint.f64 %0, [%1], %2;" : "=d"(v) : "l"(p), "l"(policy));
+      return v;
+    }
+  }
+};
+
 // Programmatic dependent launch. pdl_enter() at the top of a kernel waits
 // until the grid it depends on has completed and its writes are visible (a
 // no-op unless the kernel was launched with the programmatic-serialization
@@ -138,6 +169,20 @@ inline cudaError_t validate_domain(bool any_null, unsigned bx, unsigned by, unsi
   g.tiles = (int)((cells + g.bx - 1) / g.bx);
   g.by_nx = FastDiv((unsigned)nx);
   return cudaSuccess;
+}
+
+// Whether the loads of a step mark their lines to be evicted first. Each
+// population is read once per step, so when the buffers read and written (bytes
+// in all) only just exceed the L2 (126 MB), giving up the lines already read
+// keeps those being written, which the next step reads. Below that everything
+// stays in L2 anyway; above it little does, and the reuse of a line by the
+// neighbouring rows suffers. One step in us without and with it: D3Q19 FP64
+// BGK 80^3 (156 MB) 23.2 and 17.2, D2Q9 FP64 BGK 1024^2 (151 MB) 22.1 and 15.9,
+// D3Q19 FP32 TRT 96^3 (134 MB) 21.8 and 20.2; D3Q19 FP32 TRT 112^3 (214 MB)
+// 35.5 and 36.7, 144^3 (454 MB) 71 and 80.
+constexpr size_t kL2Bytes = (size_t)126 << 20;
+inline bool evict_first_loads(size_t bytes) {
+  return bytes > kL2Bytes / 16 * 14 && bytes < kL2Bytes / 16 * 20;
 }
 
 struct Span {

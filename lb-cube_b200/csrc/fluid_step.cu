@@ -1,15 +1,12 @@
 // Fused pull-scheme collide-stream step for D2Q9 / D3Q19 / D3Q27 fluids:
 // launchers and C-ABI entry points.
 //
-// Replaces launch_step_gpu (src/lattice_cuda.cu:476-520). The kernels are the
-// one-cell-per-thread step (step_cell.cuh) and the vectorised step
-// (stream_vec.cuh); kUseVec picks between them per lattice, operator and
-// precision.
+// Replaces launch_step_gpu (src/lattice_cuda.cu:476-520). The kernels and the
+// rule that picks one are in step_cell.cuh.
 #include "collide.cuh"
 #include "common.cuh"
 #include "diag.cuh"
 #include "step_cell.cuh"
-#include "stream_vec.cuh"
 #include "../../include/lbcube_b200.h"
 
 namespace lbcube {
@@ -27,21 +24,9 @@ cudaError_t launch_fluid_step(const Real* cur, Real* nxt, size_t nx, size_t ny, 
   const Span writes[1] = {{nxt, bytes}};
   if (any_overlap(reads, writes)) return cudaErrorInvalidValue;
   const Real omega_minus = CT == kTRT ? trt_omega_minus<Real>(omega) : Real(0);
-  if constexpr (kUseVec<L, Real, CT>) {
-    using S = NativeStorage<Real, kVecCells<L, Real>>;
-    if (vec_eligible<S>(g, cur, nxt)) {
-      const VecGrid vg = make_vec_grid(g, S::V);
-      launch_vec_step<L, S, CT>(vg, vec_grid_dims(vg), vec_block_threads(vg), stream, cur, nxt,
-                                omega, omega_minus, typename S::Params{});
-      return cudaGetLastError();
-    }
-  }
-  if constexpr (kUsePlanes<L, Real, CT>)
-    return launch_pdl(fluid_step_planes_kernel<L, Real, CT>, grid_dims(g), dim3(block_dims(g)), 0, stream,
-                      planes_of<const Real, L::Q>(cur, g), planes_of<Real, L::Q>(nxt, g), g, omega,
-                      omega_minus);
-  return launch_pdl(fluid_step_kernel<L, Real, CT, false>, grid_dims(g), dim3(block_dims(g)), 0, stream,
-                    cur, nxt, g, omega, omega_minus, (double*)nullptr);
+  if (evict_first_loads(2 * bytes))
+    return launch_step<L, Real, CT, false, true>(g, g.nz, cur, nxt, omega, omega_minus, nullptr, nullptr, stream);
+  return launch_step<L, Real, CT, false, false>(g, g.nz, cur, nxt, omega, omega_minus, nullptr, nullptr, stream);
 }
 
 // One step plus the diagnostics of the state it writes (diag.cuh): the
@@ -62,23 +47,8 @@ cudaError_t launch_fluid_step_diag(const Real* cur, Real* nxt, size_t nx, size_t
   const Span writes[3] = {{nxt, bytes}, {partials, need}, {out, kDiagOut * sizeof(double)}};
   if (any_overlap(reads, writes)) return cudaErrorInvalidValue;
   const Real omega_minus = CT == kTRT ? trt_omega_minus<Real>(omega) : Real(0);
-  long long count = -1;
-  if constexpr (kUseVec<L, Real, CT>) {
-    using S = NativeStorage<Real, kVecCells<L, Real>>;
-    if (vec_eligible<S>(g, cur, nxt)) {
-      const VecGrid vg = make_vec_grid(g, S::V);
-      const dim3 grid = vec_grid_dims(vg);
-      count = (long long)grid.x * grid.y;  // <= g.blocks(): a vector block spans >= one row block
-      err = launch_pdl(fluid_step_vec_kernel<L, S, CT, true, false>, grid, dim3(vec_block_threads(vg)), 0,
-                       stream, cur, nxt, vg, omega, omega_minus, typename S::Params{}, partials,
-                       SlabArgs<Real>{});
-    }
-  }
-  if (count < 0) {
-    count = g.launched();
-    err = launch_pdl(fluid_step_kernel<L, Real, CT, true>, grid_dims(g), dim3(block_dims(g)), 0, stream, cur,
-                     nxt, g, omega, omega_minus, partials);
-  }
+  long long count = 0;
+  err = launch_step<L, Real, CT, true, false>(g, g.nz, cur, nxt, omega, omega_minus, partials, &count, stream);
   if (err != cudaSuccess) return err;
   return launch_diag_finalize(partials, count, speed_limit, out, stream);
 }

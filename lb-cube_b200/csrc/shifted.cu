@@ -13,8 +13,8 @@
 
 #include "collide.cuh"
 #include "common.cuh"
+#include "slab_faces.cuh"
 #include "stream_codes.cuh"
-#include "stream_vec.cuh"
 #include "../../include/lbcube_b200.h"
 
 namespace lbcube {
@@ -97,7 +97,7 @@ cudaError_t launch_shifted_slab_step(const void* cur_v, void* nxt_v, size_t nx, 
   if (nz == 1 && (hl == nullptr || hh == nullptr || sl == nullptr || sh == nullptr))
     return cudaErrorInvalidDevicePointer;
   const size_t bytes = (size_t)L::Q * g.plane * sizeof(E);
-  const size_t hbytes = (size_t)zcount<L>() * g.ny * g.nx * sizeof(E);
+  const size_t hbytes = (size_t)face_planes<L>() * g.ny * g.nx * sizeof(E);
   const Span reads[3] = {{cur, bytes}, {hl, hl ? hbytes : 0}, {hh, hh ? hbytes : 0}};
   const Span writes[3] = {{nxt, bytes}, {sl, sl ? hbytes : 0}, {sh, sh ? hbytes : 0}};
   if (any_overlap(reads, writes)) return cudaErrorInvalidValue;
@@ -108,7 +108,7 @@ cudaError_t launch_shifted_slab_step(const void* cur_v, void* nxt_v, size_t nx, 
     if ((uintptr_t)q % 8 != 0) return cudaErrorInvalidValue;
   const float omega_minus = CT == kTRT ? trt_omega_minus<float>(omega) : 0.0f;
   const typename S::Params p{rho0};
-  const SlabArgs<E> faces{hl, hh, sl, sh, 0};
+  const SlabArgs<E> faces{hl, hh, sl, sh};
   const int ib = (int)std::max<size_t>(z_begin, 1), ie = (int)std::min<size_t>(z_end, nz - 1);
   if (ib < ie)
     launch_code_step<L, S, CT>(g, stream, cur, nxt, omega, omega_minus, p, ib, ie - ib);

@@ -3,11 +3,11 @@
 // No reference counterpart (the reference runs one domain on one device). The
 // box is cut into slabs along z; each rank owns nz_local planes in the
 // reference's [Q, Z, Y, X] layout and steps them with the same kernels as the
-// periodic box (kUseVec, step_cell.cuh), except that the populations crossing
-// a slab face are pulled from halo planes (SlabArgs, stream_vec.cuh) and the
+// periodic box (step_cell.cuh), except that the populations crossing
+// a slab face are pulled from halo planes (slab_faces.cuh) and the
 // ones leaving through a face are also stored, in the same pass, into send
 // planes for the neighbour. One exchange per step moves the send planes into
-// the neighbours' halo planes (zcount<L>() of Q populations per face: 5 of 19
+// the neighbours' halo planes (face_planes<L>() of Q populations per face: 5 of 19
 // for D3Q19, 9 of 27 for D3Q27); the host side runs it on NCCL point-to-point
 // (lb-cube_b200/slab.py). Every cell does the arithmetic of the periodic step,
 // so a box stepped as slabs is bit-identical to the box stepped whole.
@@ -20,11 +20,31 @@
 
 #include "collide.cuh"
 #include "common.cuh"
+#include "slab_faces.cuh"
 #include "step_cell.cuh"
-#include "stream_vec.cuh"
 #include "../../include/lbcube_b200.h"
 
 namespace lbcube {
+
+// Planes g.z0 + k * g.zs of a slab with its face buffers.
+template <class L, class Real, int CT>
+__global__ void __launch_bounds__(kThreads)
+    slab_face_kernel(const Real* __restrict__ cur, Real* __restrict__ nxt, Grid g, Real omega,
+                     Real omega_minus, SlabArgs<Real> slab) {
+  pdl_enter();
+  int x, y, z;
+  if (!cell_of(g, x, y, z)) return;
+  Real f[L::Q];
+  gather_slab<L>(cur, g, neighbours(g, x, y, z), x, y, z, slab.halo_lo, slab.halo_hi, f);
+  collide<L, Real, CT>(f, omega, omega_minus);
+  store_cell<L>(nxt, g, (z * g.ny + y) * g.nx + x, f);
+  send_slab<L>(g, x, y, z, f, slab.send_lo, slab.send_hi);
+}
+
+// The public contract of the slab step: FP32 D3Q19 rows of an even length in
+// 8-byte aligned buffers, any row of aligned elements otherwise.
+template <class L, class Real>
+constexpr int kSlabCells = (sizeof(Real) == 4 && L::Q != 27) ? 2 : 1;
 
 template <class L, class Real, int CT>
 cudaError_t launch_slab_step(const Real* cur, Real* nxt, size_t nx, size_t ny, size_t nz,
@@ -41,50 +61,36 @@ cudaError_t launch_slab_step(const Real* cur, Real* nxt, size_t nx, size_t ny, s
   // a face plane reads both halos when nz == 1
   if (nz == 1 && (halo_lo == nullptr || halo_hi == nullptr || send_lo == nullptr || send_hi == nullptr))
     return cudaErrorInvalidDevicePointer;
-  using S = NativeStorage<Real, kVecCells<L, Real>>;  // as the periodic step
-  if (!vec_eligible<S>(g, cur, nxt)) return cudaErrorInvalidValue;
+  constexpr uintptr_t align = sizeof(Real) * kSlabCells<L, Real>;
+  if (g.nx % kSlabCells<L, Real> != 0) return cudaErrorInvalidValue;
+  for (const void* p : {(const void*)cur, (const void*)nxt})
+    if ((uintptr_t)p % align != 0) return cudaErrorInvalidValue;
   const size_t bytes = (size_t)L::Q * g.plane * sizeof(Real);
-  const size_t hbytes = (size_t)zcount<L>() * g.ny * g.nx * sizeof(Real);
+  const size_t hbytes = (size_t)face_planes<L>() * g.ny * g.nx * sizeof(Real);
   const Span reads[3] = {{cur, bytes}, {halo_lo, halo_lo ? hbytes : 0}, {halo_hi, halo_hi ? hbytes : 0}};
   const Span writes[3] = {{nxt, bytes}, {send_lo, send_lo ? hbytes : 0}, {send_hi, send_hi ? hbytes : 0}};
   if (any_overlap(reads, writes)) return cudaErrorInvalidValue;
-  constexpr uintptr_t align = sizeof(Real) * S::V;
   for (const void* p : {(const void*)halo_lo, (const void*)halo_hi, (const void*)send_lo, (const void*)send_hi})
     if ((uintptr_t)p % align != 0) return cudaErrorInvalidValue;
   const Real omega_minus = CT == kTRT ? trt_omega_minus<Real>(omega) : Real(0);
-  VecGrid vg = make_vec_grid(g, S::V);
   // Interior planes [1, nz - 1) of the range pull only within the slab (no
-  // wrap) and send nothing: the periodic-box kernel that the plain step uses
-  // for this lattice, operator and precision (kUseVec) steps them, from plane
-  // z0 on. Only the face planes run the SLAB form (halo rows, face sends),
-  // whose extra addressing and stores cost about 30 % per plane.
+  // wrap) and send nothing: the periodic-box kernel steps them, from plane z0
+  // on. Only the face planes run the slab form (halo rows, face sends), whose
+  // extra addressing and stores cost about 30 % per plane.
   const size_t ib = std::max<size_t>(z_begin, 1), ie = std::min<size_t>(z_end, nz - 1);
   if (ib < ie) {
-    if constexpr (kUseVec<L, Real, CT>) {
-      vg.z0 = (int)ib;
-      dim3 grid = vec_grid_dims(vg);
-      grid.y = (unsigned)(ie - ib);
-      launch_vec_step<L, S, CT>(vg, grid, vec_block_threads(vg), s, cur, nxt, omega, omega_minus,
-                                typename S::Params{});
-      vg.z0 = 0;
-    } else {
-      Grid gi = g;
-      gi.z0 = (int)ib;
-      dim3 grid = grid_dims(gi);
-      grid.y = (unsigned)(ie - ib);
-      launch_pdl(fluid_step_kernel<L, Real, CT, false>, grid, dim3(block_dims(gi)), 0, s, cur, nxt, gi,
-                 omega, omega_minus, (double*)nullptr);
-    }
+    Grid gi = g;
+    gi.z0 = (int)ib;
+    launch_step<L, Real, CT, false, false>(gi, (int)(ie - ib), cur, nxt, omega, omega_minus, nullptr, nullptr, s);
   }
   // the face planes: `count` planes from z, `step` apart (both faces of the
   // slab in one launch where the range has both)
   auto faces = [&](size_t z, unsigned count, int step) {
-    dim3 grid = vec_grid_dims(vg);
-    grid.y = count;
-    SlabArgs<Real> slab{halo_lo, halo_hi, send_lo, send_hi, (int)z};
-    slab.z_step = step;
-    launch_pdl(fluid_step_vec_kernel<L, S, CT, false, true>, grid, dim3(vec_block_threads(vg)), 0, s, cur,
-               nxt, vg, omega, omega_minus, typename S::Params{}, (double*)nullptr, slab);
+    Grid gf = g;
+    gf.z0 = (int)z;
+    gf.zs = step;
+    launch_pdl(slab_face_kernel<L, Real, CT>, dim3((unsigned)g.tiles, count), dim3(block_dims(g)), 0, s, cur, nxt,
+               gf, omega, omega_minus, SlabArgs<Real>{halo_lo, halo_hi, send_lo, send_hi});
   };
   if (lo_face && hi_face && nz > 1) {
     faces(0, 2, (int)nz - 1);
@@ -102,7 +108,7 @@ __global__ void __launch_bounds__(256)
     slab_pack_kernel(const Real* __restrict__ f, Real* __restrict__ send_lo,
                      Real* __restrict__ send_hi, int nx, int ny, int nz) {
   const long long n2 = (long long)nx * ny;
-  const long long total = (long long)zcount<L>() * n2;
+  const long long total = (long long)face_planes<L>() * n2;
   for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total;
        e += (long long)gridDim.x * blockDim.x) {
     const int k = (int)(e / n2);
@@ -111,9 +117,9 @@ __global__ void __launch_bounds__(256)
       constexpr int i = LB_I(I);
       constexpr int cz = L::c[i][2];
       if constexpr (cz > 0) {
-        if (zslot<L>(i) == k) send_hi[e] = f[(size_t)i * n2 * nz + (size_t)(nz - 1) * n2 + r];
+        if (zslot_of<L>(i) == k) send_hi[e] = f[(size_t)i * n2 * nz + (size_t)(nz - 1) * n2 + r];
       } else if constexpr (cz < 0) {
-        if (zslot<L>(i) == k) send_lo[e] = f[(size_t)i * n2 * nz + r];
+        if (zslot_of<L>(i) == k) send_lo[e] = f[(size_t)i * n2 * nz + r];
       }
     });
   }
@@ -126,11 +132,11 @@ cudaError_t launch_slab_pack(const Real* f, size_t nx, size_t ny, size_t nz, Rea
   cudaError_t err = validate_domain(f == nullptr || send_lo == nullptr || send_hi == nullptr, 1, 1,
                                     1, 3, nx, ny, nz, g);
   if (err != cudaSuccess) return err;
-  const size_t hbytes = (size_t)zcount<L>() * g.ny * g.nx * sizeof(Real);
+  const size_t hbytes = (size_t)face_planes<L>() * g.ny * g.nx * sizeof(Real);
   const Span reads[1] = {{f, (size_t)L::Q * g.plane * sizeof(Real)}};
   const Span writes[2] = {{send_lo, hbytes}, {send_hi, hbytes}};
   if (any_overlap(reads, writes)) return cudaErrorInvalidValue;
-  const long long total = (long long)zcount<L>() * g.nx * g.ny;
+  const long long total = (long long)face_planes<L>() * g.nx * g.ny;
   const int blocks = (int)std::min<long long>((total + 255) / 256, 148LL * 16);
   slab_pack_kernel<L, Real><<<blocks, 256, 0, s>>>(f, send_lo, send_hi, g.nx, g.ny, g.nz);
   return cudaGetLastError();
@@ -172,8 +178,8 @@ cudaError_t slab_by_collision(int lattice, int collision, const void* cur, void*
 using namespace lbcube;
 
 extern "C" size_t lbm_slab_face_elems(int lattice, size_t x_extent, size_t y_extent) {
-  if (lattice == LBM_D3Q19) return (size_t)zcount<D3Q19>() * x_extent * y_extent;
-  if (lattice == LBM_D3Q27) return (size_t)zcount<D3Q27>() * x_extent * y_extent;
+  if (lattice == LBM_D3Q19) return (size_t)face_planes<D3Q19>() * x_extent * y_extent;
+  if (lattice == LBM_D3Q27) return (size_t)face_planes<D3Q27>() * x_extent * y_extent;
   return 0;
 }
 

@@ -3,7 +3,7 @@
 // steps one periodic box on one device.
 //
 // A rank owns planes [0, nz) of a box cut along z (slab.cu holds the fluid
-// alone). One face buffer per side holds, per crossing population in
+// alone, whose face buffers are the fluid part of these). One face buffer per side holds, per crossing population in
 // ascending i, an ny x nx plane: first the fluid's (5 of 19 for D3Q19, 9 of 27
 // for D3Q27), then species A's and B's (1 of 7 each for D3Q7).
 // * gather_slab (forward pull): populations with c_z = +1 at plane 0 come
@@ -25,6 +25,15 @@
 #include "lattices.cuh"
 
 namespace lbcube {
+
+// The face buffers of a slab step (elements E: a precision or 16-bit codes).
+template <class E>
+struct SlabArgs {
+  const E* halo_lo;  // c_z = +1 populations of the lower neighbour's top plane
+  const E* halo_hi;  // c_z = -1 populations of the upper neighbour's bottom plane
+  E* send_lo;        // this step's c_z = -1 populations of plane 0 (for the lower neighbour)
+  E* send_hi;        // this step's c_z = +1 populations of plane nz - 1 (for the upper one)
+};
 
 template <class L>
 __host__ __device__ constexpr int face_planes() {

@@ -1,24 +1,26 @@
-// One-cell-per-thread fused pull-scheme collide-stream step for D2Q9 / D3Q19 /
-// D3Q27 fluids, and the rule that picks it over the vectorised kernel
-// (stream_vec.cuh); shared by the periodic step (fluid_step.cu) and the
-// interior planes of the slab step (slab.cu).
+// Fused pull-scheme collide-stream step for D2Q9 / D3Q19 / D3Q27 fluids: one
+// cell per thread, and two FP32 cells per thread (pairs.cuh); shared by the
+// periodic step (fluid_step.cu) and the interior planes of the slab step
+// (slab.cu).
 //
-// Replaces kernel_step (src/lattice_cuda.cu:149-213). One thread owns one
-// destination cell: it gathers the Q incoming populations f_i(x - c_i) from
-// the current buffer (periodic wrap by compare-and-select on 32-bit
-// coordinates instead of the reference's 64-bit modulo), collides in registers
-// and writes the Q results to the next buffer at its own cell. A warp covers 32
-// consecutive x cells, so each of the Q gathers and Q stores is one coalesced
-// 128-byte row segment (shifted by at most one element for c_x != 0, which the
+// Replaces kernel_step (src/lattice_cuda.cu:149-213). In the one-cell form a
+// thread owns one destination cell: it gathers the Q incoming populations
+// f_i(x - c_i) from the current buffer (periodic wrap by compare-and-select on
+// 32-bit coordinates instead of the reference's 64-bit modulo), collides in
+// registers and writes the Q results to the next buffer at its own cell. A warp
+// covers 32 consecutive cells, so each of the Q gathers and Q stores is one
+// coalesced segment (shifted by at most one element for c_x != 0, which the
 // L1/L2 sector reuse absorbs). Planes g.z0 + k * g.zs (k < gridDim.y) are stepped.
 #pragma once
 #include "collide.cuh"
 #include "common.cuh"
 #include "diag.cuh"
+#include "pairs.cuh"
 
 namespace lbcube {
 
-template <class L, class Real, int CT>
+// FIRST: evict_first_loads.
+template <class L, class Real, int CT, bool FIRST>
 __device__ __forceinline__ void step_cell(const Real* __restrict__ cur, Real* __restrict__ nxt,
                                           const Grid& g, int x, int y, int z, Real omega,
                                           Real omega_minus, Real (&f)[L::Q]) {
@@ -26,6 +28,7 @@ __device__ __forceinline__ void step_cell(const Real* __restrict__ cur, Real* __
   const int ym = y == 0 ? g.ny - 1 : y - 1, yp = y == g.ny - 1 ? 0 : y + 1;
   const int zm = z == 0 ? g.nz - 1 : z - 1, zp = z == g.nz - 1 ? 0 : z + 1;
   const size_t plane = (size_t)g.plane;
+  const PullLoad<FIRST> load;
 
   static_for<L::Q>([&](auto I) {
     constexpr int i = LB_I(I);
@@ -34,7 +37,7 @@ __device__ __forceinline__ void step_cell(const Real* __restrict__ cur, Real* __
     const int sx = cx == 0 ? x : (cx > 0 ? xm : xp);
     const int sy = cy == 0 ? y : (cy > 0 ? ym : yp);
     const int sz = cz == 0 ? z : (cz > 0 ? zm : zp);
-    f[i] = __ldg(cur + plane * i + ((sz * g.ny + sy) * g.nx + sx));
+    f[i] = load(cur + plane * i + ((sz * g.ny + sy) * g.nx + sx));
   });
 
   collide<L, Real, CT>(f, omega, omega_minus);
@@ -47,11 +50,12 @@ __device__ __forceinline__ void step_cell(const Real* __restrict__ cur, Real* __
 }
 
 // DIAG: also reduce the diagnostics of the written state over the block
-// (diag.cuh), as in fluid_step_vec_kernel.
-template <class L, class Real, int CT, bool DIAG = false>
+// (diag.cuh): in the pull scheme the populations a thread writes are exactly the
+// next buffer's populations of its own cell, so this costs no memory traffic.
+template <class L, class Real, int CT, bool DIAG, bool FIRST>
 __global__ void __launch_bounds__(kThreads)
     fluid_step_kernel(const Real* __restrict__ cur, Real* __restrict__ nxt, Grid g, Real omega,
-                      Real omega_minus, double* __restrict__ partials = nullptr) {
+                      Real omega_minus, double* __restrict__ partials) {
   pdl_enter();
   int x, y, z;
   const bool active = cell_of(g, x, y, z);
@@ -59,13 +63,13 @@ __global__ void __launch_bounds__(kThreads)
   if constexpr (DIAG) {
     DiagAcc acc;
     if (active) {
-      step_cell<L, Real, CT>(cur, nxt, g, x, y, z, omega, omega_minus, f);
+      step_cell<L, Real, CT, FIRST>(cur, nxt, g, x, y, z, omega, omega_minus, f);
       diag_cell<L>(f, acc);
     }
     diag_block_to(acc, partials + block_linear() * kDiagPartials);
   } else {
     if (!active) return;
-    step_cell<L, Real, CT>(cur, nxt, g, x, y, z, omega, omega_minus, f);
+    step_cell<L, Real, CT, FIRST>(cur, nxt, g, x, y, z, omega, omega_minus, f);
   }
 }
 
@@ -76,13 +80,9 @@ __global__ void __launch_bounds__(kThreads)
 // D3Q27, where it measured faster (A/B, same box, bit-identical outputs:
 // D3Q19 FP64 MRT 0.94 -> 0.98 of the copy bandwidth at 256^3, D3Q27 FP32 MRT
 // 0.56 -> 0.585 at 224^3; D3Q19 FP32 MRT and D3Q27 BGK level; RLBM 1.5-7 % and
-// D2Q9 MRT 2.5 % slower, so those keep fluid_step_kernel). LBCUBE_PLANE_PTRS = 0
-// turns it off.
-#ifndef LBCUBE_PLANE_PTRS
-#define LBCUBE_PLANE_PTRS 1
-#endif
+// D2Q9 MRT 2.5 % slower, so those keep fluid_step_kernel).
 template <class L, class Real, int CT>
-constexpr bool kUsePlanes = LBCUBE_PLANE_PTRS != 0 && CT == kMRT && L::Q >= 19;
+constexpr bool kUsePlanes = CT == kMRT && L::Q >= 19;
 template <class Real, int Q>
 struct Planes {
   Real* p[Q];
@@ -96,7 +96,7 @@ inline Planes<Real, Q> planes_of(Real* base, const Grid& g) {
 
 // fluid_step_kernel (no diagnostics) on plane pointers: the same gather,
 // collision and stores, so the same bits.
-template <class L, class Real, int CT>
+template <class L, class Real, int CT, bool FIRST>
 __global__ void __launch_bounds__(kThreads)
     fluid_step_planes_kernel(const Planes<const Real, L::Q> cur, const Planes<Real, L::Q> nxt,
                              Grid g, Real omega, Real omega_minus) {
@@ -107,41 +107,95 @@ __global__ void __launch_bounds__(kThreads)
   const int ym = y == 0 ? g.ny - 1 : y - 1, yp = y == g.ny - 1 ? 0 : y + 1;
   const int zm = z == 0 ? g.nz - 1 : z - 1, zp = z == g.nz - 1 ? 0 : z + 1;
   Real f[L::Q];
+  const PullLoad<FIRST> load;
   static_for<L::Q>([&](auto I) {
     constexpr int i = LB_I(I);
     constexpr int cx = L::c[i][0], cy = L::c[i][1], cz = L::c[i][2];
     const int sx = cx == 0 ? x : (cx > 0 ? xm : xp);
     const int sy = cy == 0 ? y : (cy > 0 ? ym : yp);
     const int sz = cz == 0 ? z : (cz > 0 ? zm : zp);
-    f[i] = __ldg(cur.p[i] + ((sz * g.ny + sy) * g.nx + sx));
+    f[i] = load(cur.p[i] + ((sz * g.ny + sy) * g.nx + sx));
   });
   collide<L, Real, CT>(f, omega, omega_minus);
   const int cell = (z * g.ny + y) * g.nx + x;
   static_for<L::Q>([&](auto I) { nxt.p[LB_I(I)][cell] = f[LB_I(I)]; });
 }
 
-// Cells per thread of the vectorised kernel, measured fastest on B200 at 256^3:
-// 2 FP32 D2Q9 / D3Q19 cells (8-byte words; D3Q19 TRT 0.99 of the copy
-// bandwidth against 0.80 at V = 4 and 0.76 at V = 1), 1 D3Q27 FP32 cell (BGK
-// 0.86 against 0.75 at V = 2, TRT 0.80 against 0.58) and 1 FP64 cell.
-// The plain step of native storage runs the vectorised kernel only for FP32
-// D3Q19 BGK and TRT, where it is level with the one-cell kernel; every other
-// lattice, operator and precision measured faster with the one-cell kernel
-// (A/B at 256^3 / 4096^2, bitwise-identical outputs, fraction of the copy
-// bandwidth): D3Q27 FP32 BGK 0.76 -> 0.97, TRT 0.74 -> 0.95, MRT 0.48 -> 0.56,
-// RLBM 0.59 -> 0.68; D3Q27 FP64 BGK 0.91 -> 1.03, TRT 0.88 -> 1.03; D3Q19 FP32
-// MRT 0.80 -> 0.87; D3Q19 FP64 MRT 0.86 -> 0.97, RLBM 0.74 -> 0.84; D2Q9 FP32
-// 2-5 % and FP64 4-18 %. Two cells per thread double the live populations
-// (D3Q19 FP32 MRT: 80 registers against 40); at one cell per thread (D3Q27
-// FP32, FP64) both kernels hold the same values, and they differ in the
-// gather: the vectorised kernel exchanges x-neighbours by warp shuffles with
-// extra loads at the warp edges, the one-cell kernel loads every neighbour
-// directly (overlapping row segments, served by L1).
-// The slab step follows the same rule on its interior planes; its face planes
-// and the 16-bit storage keep the vectorised kernel.
-template <class L, class Real>
-constexpr int kVecCells = (sizeof(Real) == 4 && L::Q != 27) ? 2 : 1;
+// ---- two FP32 cells per thread ---------------------------------------------------
+// One step in us, one cell per thread -> two: D3Q19 TRT 256^3 394 -> 380 (6.7 TB/s,
+// a copy's rate), 160^3 100 -> 97, 96^3 22.1 -> 20.4; MRT 128^3 59 -> 55; RLBM
+// 128^3 69 -> 60; D3Q27 BGK 128^3 74 -> 72, RLBM 105 -> 95; D2Q9 BGK 1448^2 24.7 ->
+// 20.5. Against the kernel that exchanged x-neighbours by shuffles, a warp per
+// row: D3Q19 TRT 256^3 383, 160^3 118, 96^3 29.7. Four cells per thread: level
+// at 256^3, slower below.
+//
+// Resident blocks of kThreads per SM that the register allocation must allow
+// (0: the compiler's choice): D3Q19 7 (72 registers; TRT 180 x 170 x 190 140 us
+// against 143 at 6 and 142 at 8; MRT 151, 159 and 154), RLBM, D2Q9 and D3Q27 the
+// compiler's (D3Q27 BGK 72 x 70 x 68 9.8 us against 11.0 at 4).
+template <class L, int CT>
+constexpr int kPairBlocks = L::Q == 19 && CT != kRLBM ? 7 : 0;
+// Not the D3Q27 MRT, whose 54 populations and as many moments leave too few
+// warps (72 x 70 x 68 16.4 -> 18.6 us).
 template <class L, class Real, int CT>
-constexpr bool kUseVec = sizeof(Real) == 4 && L::Q == 19 && (CT == kBGK || CT == kTRT);
+constexpr bool kUsePairs = sizeof(Real) == 4 && !(L::Q == 27 && CT == kMRT);
+// From how many one-cell blocks per SM on (pairs_eligible): what the SMs hold
+// at once. D3Q19 12: MRT 56^3 (9.3 blocks per SM) 6.6 -> 7.1 us, 64^3 (13.8) 7.7 ->
+// 6.8. D2Q9 16: MRT 512^2 (13.8) 4.2 -> 5.2, 600^2 (19) 5.1 -> 5.0, 724^2 6.5 -> 5.8.
+// D3Q27 likewise: BGK 64^3 (13.8) level, 72^3 (19.7) 11.5 -> 10.4; its RLBM later:
+// 72^3 18.0 -> 18.4, 88^3 (36) 36.6 -> 33.7.
+template <class L, int CT>
+constexpr int kPairFrom = L::Q == 19 ? 12 : L::Q == 27 && CT == kRLBM ? 30 : 16;
+
+template <class L, int CT, bool DIAG, bool FIRST>
+__global__ void __launch_bounds__(kThreads, kPairBlocks<L, CT>)
+    fluid_step_pair_kernel(const float* __restrict__ cur, float* __restrict__ nxt, PairGrid g, float omega,
+                           float omega_minus, double* __restrict__ partials) {
+  pdl_enter();
+  int x0, y, z;
+  const bool active = pair_of(g, x0, y, z);
+  DiagAcc acc;
+  if (active) {
+    float f[2][L::Q];
+    gather_pair<L, FIRST>(cur, g, PairRows(g, x0, y, z), f);
+#pragma unroll
+    for (int j = 0; j < 2; ++j) collide<L, float, CT>(f[j], omega, omega_minus);
+    store_pair(nxt, g, (z * g.ny + y) * g.nx + x0, f);
+    if constexpr (DIAG) {
+#pragma unroll
+      for (int j = 0; j < 2; ++j) diag_cell<L>(f[j], acc);
+    }
+  }
+  if constexpr (DIAG)
+    diag_block_to(acc, partials + ((long long)blockIdx.y * gridDim.x + blockIdx.x) * kDiagPartials);
+}
+
+// One step of planes g.z0 .. g.z0 + planes - 1 on the kernel that is the faster one
+// for this lattice, operator, precision and row length. DIAG: with the
+// diagnostics' partials, whose count goes to *count (over every plane; at most
+// g.launched()).
+template <class L, class Real, int CT, bool DIAG, bool FIRST>
+inline cudaError_t launch_step(const Grid& g, int planes, const Real* cur, Real* nxt, Real omega,
+                               Real omega_minus, double* partials, long long* count, cudaStream_t s) {
+  // programmatic dependent launches (the kernels open with pdl_enter)
+  if constexpr (kUsePairs<L, Real, CT>) {
+    if (pairs_eligible(g, kPairFrom<L, CT>, cur, nxt)) {
+      const PairGrid pg = make_pair_grid(g, g.z0);
+      const dim3 grid = pair_grid_dims(pg, planes);
+      if constexpr (DIAG) *count = (long long)grid.x * planes;
+      return launch_pdl(fluid_step_pair_kernel<L, CT, DIAG, FIRST>, grid, dim3(kThreads), 0, s, cur, nxt, pg,
+                        omega, omega_minus, partials);
+    }
+  }
+  const dim3 grid((unsigned)g.tiles, (unsigned)planes), block(block_dims(g));
+  if constexpr (DIAG) *count = (long long)g.tiles * planes;
+  if constexpr (kUsePlanes<L, Real, CT> && !DIAG)
+    return launch_pdl(fluid_step_planes_kernel<L, Real, CT, FIRST>, grid, block, 0, s,
+                      planes_of<const Real, L::Q>(cur, g), planes_of<Real, L::Q>(nxt, g), g, omega,
+                      omega_minus);
+  else
+    return launch_pdl(fluid_step_kernel<L, Real, CT, DIAG, FIRST>, grid, block, 0, s, cur, nxt, g, omega,
+                      omega_minus, partials);
+}
 
 }  // namespace lbcube

@@ -28,9 +28,9 @@
 
 #include <cstdint>
 
-#include "collide_dev.cuh"
+#include "codes.cuh"
 #include "common.cuh"
-#include "stream_vec.cuh"
+#include "slab_faces.cuh"
 
 namespace lbcube {
 
@@ -111,9 +111,9 @@ __device__ __forceinline__ void gather_words(const unsigned short* __restrict__ 
     const int sz = cz == 0 ? z : (cz > 0 ? zm : zp);
     const unsigned short* row = cur + plane * i + (unsigned int)((sz * g.ny + sy) * g.nx);
     if constexpr (SLAB && cz > 0) {
-      if (z == 0) row = slab.halo_lo + (size_t)(zslot<L>(i) * g.ny + sy) * g.nx;
+      if (z == 0) row = slab.halo_lo + (size_t)(zslot_of<L>(i) * g.ny + sy) * g.nx;
     } else if constexpr (SLAB && cz < 0) {
-      if (z == g.nz - 1) row = slab.halo_hi + (size_t)(zslot<L>(i) * g.ny + sy) * g.nx;
+      if (z == g.nz - 1) row = slab.halo_hi + (size_t)(zslot_of<L>(i) * g.ny + sy) * g.nx;
     }
     pull_codes<cx>(row, x0, xl, xr, raw[i]);
   });
@@ -153,9 +153,9 @@ __device__ __forceinline__ void code_step_body(const unsigned short* __restrict_
     // the populations leaving through a face, at the cells' own (x, y)
     if constexpr (SLAB && cz > 0) {
       if (z == g.nz - 1)
-        *reinterpret_cast<uint2*>(slab.send_hi + (size_t)(zslot<L>(i) * g.ny + y) * g.nx + x0) = w;
+        *reinterpret_cast<uint2*>(slab.send_hi + (size_t)(zslot_of<L>(i) * g.ny + y) * g.nx + x0) = w;
     } else if constexpr (SLAB && cz < 0) {
-      if (z == 0) *reinterpret_cast<uint2*>(slab.send_lo + (size_t)(zslot<L>(i) * g.ny + y) * g.nx + x0) = w;
+      if (z == 0) *reinterpret_cast<uint2*>(slab.send_lo + (size_t)(zslot_of<L>(i) * g.ny + y) * g.nx + x0) = w;
     }
   });
 }
