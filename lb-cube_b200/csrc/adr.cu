@@ -7,12 +7,14 @@
 //                       (src/simulate_reaction.cpp:518-543), optionally with
 //                       the reactive-statistics partial sums of the new fields.
 #include <algorithm>
+#include <type_traits>
 
 #include "adr.cuh"
 #include "slab_faces.cuh"
 #include "cells.cuh"
 #include "collide.cuh"
 #include "common.cuh"
+#include "pairs.cuh"
 #include "reduce.cuh"
 #include "../../include/lbcube_b200.h"
 
@@ -120,22 +122,146 @@ __global__ void __launch_bounds__(kThreads)
                                                  omega_minus, omega_c, k, partials, u_out);
 }
 
-// The statistics form of the FP32 D2Q9 step with the plain step's register
-// budget (LBCUBE_STATS_MIN_BLOCKS resident blocks per SM): its FP64 sums and
-// block reduction otherwise take 46 registers instead of 40, two resident
-// blocks fewer (1024^2: 33.6 instead of 35.0 us per launch).
-#ifndef LBCUBE_STATS_MIN_BLOCKS
-#define LBCUBE_STATS_MIN_BLOCKS 12
-#endif
-template <class FL, class Real, int CT>
-__global__ void __launch_bounds__(kThreads, LBCUBE_STATS_MIN_BLOCKS)
-    fluid_reaction_stats_kernel(const Real* __restrict__ cur_f, Real* __restrict__ nxt_f,
-                                const Real* __restrict__ cur_a, Real* __restrict__ nxt_a,
-                                const Real* __restrict__ cur_b, Real* __restrict__ nxt_b, Grid g,
-                                Real omega, Real omega_minus, Real omega_c, Real k,
-                                double* __restrict__ partials) {
-  fluid_reaction_body<FL, Real, CT, true, false>(cur_f, nxt_f, cur_a, nxt_a, cur_b, nxt_b, g, omega,
-                                                 omega_minus, omega_c, k, partials, nullptr);
+// ---- two FP32 cells per thread (pairs.cuh) ----------------------------------------
+// Each cell's arithmetic is that of the one-cell kernels, so are the bits. One
+// step in us, one cell -> two: coupled D2Q9 TRT 1024^2 27.9 -> 22.6 (of which the
+// evict-first loads 2.7), 2048^2 108 -> 99, D3Q19 TRT 80^3 23.3 -> 18.8, 128^3 91 -> 88; fluid and
+// scalar step D3Q19 96^3 47 -> 35, 128^3 101 -> 93; fluid and reaction 128^3 121 -> 111.
+
+// Resident blocks of kThreads per SM that the register allocation must allow
+// (0: the compiler's choice): D3Q19 7 (64^3 9.5 us, 10.5 at 6, 10.1 at 5), D2Q9 the
+// compiler's (1024^2 with statistics every 5 steps 24.1 us, 24.4 at 8, 24.7 at 10).
+template <class FL>
+constexpr int kCoupledPairBlocks = FL::Q == 19 ? 7 : 0;
+// D2Q9 and D3Q19 only (D3Q27 96^3: 101 -> 113 us), from the box on whose one-cell
+// launch no longer fits the SMs at once (pairs_eligible): D2Q9 512^2 7.0 -> 7.2,
+// 640^2 9.5 -> 8.8 us; D3Q19 40^3 5.1 -> 5.7, 64^3 10.3 -> 9.5 us.
+template <class FL, class Real>
+constexpr bool kAdrPairs = std::is_same_v<Real, float> && FL::Q <= 19;
+template <class FL>
+constexpr int kAdrPairFrom = FL::Q == 19 ? 12 : 16;
+
+template <class FL>
+__global__ void __launch_bounds__(kThreads)
+    scalar_step_pair_kernel(const float* __restrict__ cur_s, float* __restrict__ nxt_s,
+                            const float* __restrict__ cur_f, PairGrid g, float omega_c, float source) {
+  using SL = typename ScalarOf<FL>::type;
+  pdl_enter();
+  int x0, y, z;
+  if (!pair_of(g, x0, y, z)) return;
+  const int cell = (z * g.ny + y) * g.nx + x0;
+  float f[2][FL::Q], u[2][FL::D], s[2][SL::Q];
+  load_pair<FL>(cur_f, g, cell, f);
+  gather_pair<SL>(cur_s, g, PairRows(g, x0, y, z), s);
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    fluid_velocity<FL>(f[j], u[j]);
+    collide_scalar<SL>(s[j], u[j], omega_c, source);
+  }
+  store_pair(nxt_s, g, cell, s);
+}
+
+template <class FL>
+__global__ void __launch_bounds__(kThreads)
+    reaction_ab_pair_kernel(const float* __restrict__ cur_a, float* __restrict__ nxt_a,
+                            const float* __restrict__ cur_b, float* __restrict__ nxt_b,
+                            const float* __restrict__ cur_f, PairGrid g, float omega_c, float k) {
+  using SL = typename ScalarOf<FL>::type;
+  pdl_enter();
+  int x0, y, z;
+  if (!pair_of(g, x0, y, z)) return;
+  const int cell = (z * g.ny + y) * g.nx + x0;
+  float f[2][FL::Q], u[2][FL::D], a[2][SL::Q], b[2][SL::Q];
+  load_pair<FL>(cur_f, g, cell, f);
+#pragma unroll
+  for (int j = 0; j < 2; ++j) fluid_velocity<FL>(f[j], u[j]);
+  const PairRows r(g, x0, y, z);
+  gather_pair<SL>(cur_a, g, r, a);
+  gather_pair<SL>(cur_b, g, r, b);
+#pragma unroll
+  for (int j = 0; j < 2; ++j) react_pair<SL>(a[j], b[j], u[j], omega_c, k);
+  store_pair(nxt_a, g, cell, a);
+  store_pair(nxt_b, g, cell, b);
+}
+
+// STATS: the partials of the one-cell blocks that the block covers, bit for bit
+// (pair_block_sum_to), so the statistics do not depend on which kernel ran.
+template <class FL, int CT, bool STATS, bool UOUT, bool FIRST>
+__global__ void __launch_bounds__(kThreads, kCoupledPairBlocks<FL>)
+    fluid_reaction_pair_kernel(const float* __restrict__ cur_f, float* __restrict__ nxt_f,
+                               const float* __restrict__ cur_a, float* __restrict__ nxt_a,
+                               const float* __restrict__ cur_b, float* __restrict__ nxt_b, PairGrid g,
+                               float omega, float omega_minus, float omega_c, float k,
+                               double* __restrict__ partials, float* __restrict__ u_out) {
+  using SL = typename ScalarOf<FL>::type;
+  pdl_enter();
+  int x0, y, z;
+  const bool active = pair_of(g, x0, y, z);
+  double sums[2][kStatSums] = {};
+  if (active) {
+    const int cell = (z * g.ny + y) * g.nx + x0;
+    const PairRows r(g, x0, y, z);
+    float u[2][FL::D];
+    {
+      float f[2][FL::Q];
+      gather_pair<FL, FIRST>(cur_f, g, r, f);
+#pragma unroll
+      for (int j = 0; j < 2; ++j) collide<FL, float, CT>(f[j], omega, omega_minus);
+      store_pair(nxt_f, g, cell, f);
+#pragma unroll
+      for (int j = 0; j < 2; ++j) fluid_velocity<FL>(f[j], u[j]);
+    }
+    if constexpr (UOUT) store_pair(u_out, g, cell, u);
+    float a[2][SL::Q], b[2][SL::Q];
+    gather_pair<SL, FIRST>(cur_a, g, r, a);
+    gather_pair<SL, FIRST>(cur_b, g, r, b);
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      react_pair<SL>(a[j], b[j], u[j], omega_c, k);
+      if constexpr (STATS) {
+        // concentration_at of the stored fields (lattice_io.hpp:125-133)
+        const double ca = (double)concentration<SL>(a[j]), cb = (double)concentration<SL>(b[j]);
+        sums[j][0] = ca;
+        sums[j][1] = cb;
+        sums[j][2] = ca * ca;
+        sums[j][3] = cb * cb;
+        sums[j][4] = ca * cb;
+      }
+    }
+    store_pair(nxt_a, g, cell, a);
+    store_pair(nxt_b, g, cell, b);
+  }
+  if constexpr (STATS) {
+    const int first = (int)blockIdx.x * kPairCells;
+    pair_block_sum_to<kStatSums>(sums[0], sums[1], g.tiles - first,
+                                 partials + ((long long)z * g.tiles + first) * kStatSums);
+  }
+}
+
+// The coupled step of planes g.z0 .. g.z0 + planes - 1, no faces of a slab.
+template <class FL, class Real, int CT, bool STATS, bool UOUT>
+cudaError_t launch_coupled_step(const Grid& g, int planes, const Real* cur_f, Real* nxt_f, const Real* cur_a,
+                                Real* nxt_a, const Real* cur_b, Real* nxt_b, Real omega, Real omega_minus,
+                                Real omega_c, Real k, double* partials, Real* u_out, cudaStream_t s) {
+  // programmatic dependent launches (the kernels open with pdl_enter)
+  if constexpr (kAdrPairs<FL, Real>) {
+    if (pairs_eligible(g, kAdrPairFrom<FL>, cur_f, nxt_f, cur_a, nxt_a, cur_b, nxt_b, u_out)) {
+      const PairGrid pg = make_pair_grid(g, g.z0);
+      const dim3 grid = pair_grid_dims(pg, planes);
+      using SL = typename ScalarOf<FL>::type;
+      if constexpr (!UOUT) {
+        if (evict_first_loads(2 * (size_t)(FL::Q + 2 * SL::Q) * g.plane * sizeof(float)))
+          return launch_pdl(fluid_reaction_pair_kernel<FL, CT, STATS, UOUT, true>, grid, dim3(kThreads), 0, s,
+                            cur_f, nxt_f, cur_a, nxt_a, cur_b, nxt_b, pg, omega, omega_minus, omega_c, k,
+                            partials, u_out);
+      }
+      return launch_pdl(fluid_reaction_pair_kernel<FL, CT, STATS, UOUT, false>, grid, dim3(kThreads), 0, s, cur_f,
+                        nxt_f, cur_a, nxt_a, cur_b, nxt_b, pg, omega, omega_minus, omega_c, k, partials, u_out);
+    }
+  }
+  return launch_pdl(fluid_reaction_kernel<FL, Real, CT, STATS, UOUT>, dim3((unsigned)g.tiles, (unsigned)planes),
+                    dim3(block_dims(g)), 0, s, cur_f, nxt_f, cur_a, nxt_a, cur_b, nxt_b, g, omega, omega_minus,
+                    omega_c, k, partials, u_out);
 }
 
 // ---- z-slab form of the coupled step ----------------------------------------
@@ -288,11 +414,11 @@ cudaError_t launch_fluid_reaction_slab(const Real* cur_f, Real* nxt_f, const Rea
                  nxt_f, cur_a, nxt_a, cur_b, nxt_b, gr, omega, omega_minus, omega_c, k, halo_lo, halo_hi,
                  send_lo, send_hi, (double*)nullptr, none);
     else if (partials != nullptr)
-      launch_pdl(fluid_reaction_kernel<FL, Real, CT, true, false>, grid, block, 0, stream, cur_f, nxt_f,
-                 cur_a, nxt_a, cur_b, nxt_b, gr, omega, omega_minus, omega_c, k, partials, none);
+      launch_coupled_step<FL, Real, CT, true, false>(gr, planes, cur_f, nxt_f, cur_a, nxt_a, cur_b, nxt_b, omega,
+                                                     omega_minus, omega_c, k, partials, none, stream);
     else
-      launch_pdl(fluid_reaction_kernel<FL, Real, CT, false, false>, grid, block, 0, stream, cur_f, nxt_f,
-                 cur_a, nxt_a, cur_b, nxt_b, gr, omega, omega_minus, omega_c, k, (double*)nullptr, none);
+      launch_coupled_step<FL, Real, CT, false, false>(gr, planes, cur_f, nxt_f, cur_a, nxt_a, cur_b, nxt_b,
+                                                      omega, omega_minus, omega_c, k, nullptr, none, stream);
   };
   const int zb = (int)z_begin, ze = (int)z_end, last = g.nz - 1;
   const bool lo = zb == 0, hi = ze - 1 == last && last > 0 && zb <= last;
@@ -342,6 +468,13 @@ cudaError_t launch_scalar(const Real* cur_s, Real* nxt_s, const Real* cur_f, siz
   const Span reads[2] = {{cur_s, sb}, {cur_f, fb}};
   const Span writes[1] = {{nxt_s, sb}};
   if (any_overlap(reads, writes)) return cudaErrorInvalidValue;
+  if constexpr (kAdrPairs<FL, Real>) {
+    if (pairs_eligible(g, kAdrPairFrom<FL>, cur_s, nxt_s, cur_f)) {
+      const PairGrid pg = make_pair_grid(g);
+      return launch_pdl(scalar_step_pair_kernel<FL>, pair_grid_dims(pg, g.nz), dim3(kThreads), 0, stream, cur_s,
+                        nxt_s, cur_f, pg, omega_c, source);
+    }
+  }
   return launch_pdl(scalar_step_kernel<FL, Real>, grid_dims(g), dim3(block_dims(g)), 0, stream, cur_s,
                     nxt_s, cur_f, g, omega_c, source);
 }
@@ -362,6 +495,13 @@ cudaError_t launch_reaction(const Real* cur_a, Real* nxt_a, const Real* cur_b, R
   const Span reads[3] = {{cur_a, sb}, {cur_b, sb}, {cur_f, fb}};
   const Span writes[2] = {{nxt_a, sb}, {nxt_b, sb}};
   if (any_overlap(reads, writes)) return cudaErrorInvalidValue;
+  if constexpr (kAdrPairs<FL, Real>) {
+    if (pairs_eligible(g, kAdrPairFrom<FL>, cur_a, nxt_a, cur_b, nxt_b, cur_f)) {
+      const PairGrid pg = make_pair_grid(g);
+      return launch_pdl(reaction_ab_pair_kernel<FL>, pair_grid_dims(pg, g.nz), dim3(kThreads), 0, stream, cur_a,
+                        nxt_a, cur_b, nxt_b, cur_f, pg, omega_c, k);
+    }
+  }
   return launch_pdl(reaction_ab_kernel<FL, Real>, grid_dims(g), dim3(block_dims(g)), 0, stream, cur_a,
                     nxt_a, cur_b, nxt_b, cur_f, g, omega_c, k);
 }
@@ -390,20 +530,11 @@ cudaError_t launch_fluid_reaction(const Real* cur_f, Real* nxt_f, const Real* cu
     if (any_overlap(reads, writes)) return cudaErrorInvalidValue;
   }
   const Real omega_minus = CT == kTRT ? trt_omega_minus<Real>(omega) : Real(0);
-  // launched as programmatic dependents of the previous launch (pdl_enter)
-  if (partials != nullptr) {
-    if constexpr (FL::Q == 9 && sizeof(Real) == 4 && LBCUBE_STATS_MIN_BLOCKS > 0)
-      return launch_pdl(fluid_reaction_stats_kernel<FL, Real, CT>, grid_dims(g), dim3(block_dims(g)), 0,
-                        stream, cur_f, nxt_f, cur_a, nxt_a, cur_b, nxt_b, g, omega, omega_minus,
-                        omega_c, k, partials);
-    else
-      return launch_pdl(fluid_reaction_kernel<FL, Real, CT, true, false>, grid_dims(g),
-                        dim3(block_dims(g)), 0, stream, cur_f, nxt_f, cur_a, nxt_a, cur_b, nxt_b, g,
-                        omega, omega_minus, omega_c, k, partials, (Real*)nullptr);
-  }
-  return launch_pdl(fluid_reaction_kernel<FL, Real, CT, false, false>, grid_dims(g), dim3(block_dims(g)),
-                    0, stream, cur_f, nxt_f, cur_a, nxt_a, cur_b, nxt_b, g, omega, omega_minus, omega_c,
-                    k, (double*)nullptr, (Real*)nullptr);
+  if (partials != nullptr)
+    return launch_coupled_step<FL, Real, CT, true, false>(g, g.nz, cur_f, nxt_f, cur_a, nxt_a, cur_b, nxt_b,
+                                                          omega, omega_minus, omega_c, k, partials, nullptr, stream);
+  return launch_coupled_step<FL, Real, CT, false, false>(g, g.nz, cur_f, nxt_f, cur_a, nxt_a, cur_b, nxt_b, omega,
+                                                         omega_minus, omega_c, k, nullptr, nullptr, stream);
 }
 
 // The fused step with the advecting velocity stored (no statistics), for the
@@ -414,19 +545,13 @@ cudaError_t fluid_reaction_with_velocity(int collision, const Real* cur_f, Real*
                                          const Real* cur_a, Real* nxt_a, const Real* cur_b,
                                          Real* nxt_b, Real* u_out, const Grid& g, Real omega,
                                          Real omega_c, Real k, cudaStream_t s) {
-  // programmatic dependent launches (the kernel opens with pdl_enter)
-  const dim3 grid = grid_dims(g), block(block_dims(g));
-  double* const none = nullptr;
-  if (collision == kBGK)
-    return launch_pdl(fluid_reaction_kernel<FL, Real, kBGK, false, true>, grid, block, 0, s, cur_f, nxt_f,
-                      cur_a, nxt_a, cur_b, nxt_b, g, omega, Real(0), omega_c, k, none, u_out);
-  if (collision == kTRT)
-    return launch_pdl(fluid_reaction_kernel<FL, Real, kTRT, false, true>, grid, block, 0, s, cur_f, nxt_f,
-                      cur_a, nxt_a, cur_b, nxt_b, g, omega, trt_omega_minus<Real>(omega), omega_c, k,
-                      none, u_out);
-  if (collision == kMRT)
-    return launch_pdl(fluid_reaction_kernel<FL, Real, kMRT, false, true>, grid, block, 0, s, cur_f, nxt_f,
-                      cur_a, nxt_a, cur_b, nxt_b, g, omega, Real(0), omega_c, k, none, u_out);
+  auto run = [&](auto ct, Real omega_minus) {
+    return launch_coupled_step<FL, Real, decltype(ct)::value, false, true>(
+        g, g.nz, cur_f, nxt_f, cur_a, nxt_a, cur_b, nxt_b, omega, omega_minus, omega_c, k, nullptr, u_out, s);
+  };
+  if (collision == kBGK) return run(std::integral_constant<int, kBGK>{}, Real(0));
+  if (collision == kTRT) return run(std::integral_constant<int, kTRT>{}, trt_omega_minus<Real>(omega));
+  if (collision == kMRT) return run(std::integral_constant<int, kMRT>{}, Real(0));
   return cudaErrorInvalidValue;
 }
 
@@ -462,11 +587,11 @@ cudaError_t fluid_reaction_slab_with_velocity(int collision, const Real* cur_f, 
                    nxt_f, cur_a, nxt_a, cur_b, nxt_b, gr, omega, om, omega_c, k, halo_lo, halo_hi,
                    send_lo, send_hi, none, (Real*)nullptr);
       else if (u_out != nullptr)
-        launch_pdl(fluid_reaction_kernel<FL, Real, CT, false, true>, grid, block, 0, s, cur_f, nxt_f,
-                   cur_a, nxt_a, cur_b, nxt_b, gr, omega, om, omega_c, k, none, u_out);
+        launch_coupled_step<FL, Real, CT, false, true>(gr, planes, cur_f, nxt_f, cur_a, nxt_a, cur_b, nxt_b, omega,
+                                                       om, omega_c, k, none, u_out, s);
       else
-        launch_pdl(fluid_reaction_kernel<FL, Real, CT, false, false>, grid, block, 0, s, cur_f, nxt_f,
-                   cur_a, nxt_a, cur_b, nxt_b, gr, omega, om, omega_c, k, none, (Real*)nullptr);
+        launch_coupled_step<FL, Real, CT, false, false>(gr, planes, cur_f, nxt_f, cur_a, nxt_a, cur_b, nxt_b,
+                                                        omega, om, omega_c, k, none, nullptr, s);
     };
     if (g.nz >= 3) launch(1, g.nz - 2, 1, false);
     launch(0, g.nz >= 2 ? 2 : 1, g.nz - 1, true);  // both face planes in one launch

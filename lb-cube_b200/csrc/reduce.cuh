@@ -41,6 +41,39 @@ __device__ __forceinline__ void block_sum_to(double (&v)[N], double* out) {
   }
 }
 
+// The block sums of a block whose threads hold two adjacent cells each (`even`
+// and `odd` of the pair), in the order of block_sum_to: cells 128 k .. 128 k + 127
+// of the block are the one-cell block k (tiles of them, at most 2), whose warp
+// tree adds cells 16, 8, 4, 2 and 1 apart, i.e. threads 8, 4, 2 and 1 apart within
+// half a warp for either parity, then the two parities. out[k * N ..] gets the
+// totals of one-cell block k, bit for bit those of a one-cell launch.
+template <int N>
+__device__ __forceinline__ void pair_block_sum_to(double (&even)[N], double (&odd)[N], int tiles, double* out) {
+  __shared__ double part[2 * kThreads / 32][N];
+#pragma unroll
+  for (int off = 8; off > 0; off >>= 1) {
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+      even[k] += __shfl_down_sync(0xffffffffu, even[k], off, 16);
+      odd[k] += __shfl_down_sync(0xffffffffu, odd[k], off, 16);
+    }
+  }
+  if ((threadIdx.x & 15) == 0) {
+#pragma unroll
+    for (int k = 0; k < N; ++k) part[threadIdx.x >> 4][k] = even[k] + odd[k];
+  }
+  __syncthreads();
+  if ((int)threadIdx.x < min(tiles, 2)) {
+    const int w0 = 4 * (int)threadIdx.x;
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+      double s = part[w0][k];
+      for (int w = 1; w < 4; ++w) s += part[w0 + w][k];
+      out[threadIdx.x * N + k] = s;
+    }
+  }
+}
+
 // Sums v[0..N) over the warp (all 32 lanes must call it); lane 0 ends with
 // the totals. Fixed reduction tree, no block barrier.
 template <int N>
