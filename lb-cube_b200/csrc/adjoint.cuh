@@ -31,6 +31,11 @@ namespace lbcube {
 template <class Real>
 constexpr int kAdjointBlocks = sizeof(Real) == 4 ? 5 : 2;
 
+// The same for the two-cell FP32 kernels (pairs.cuh): four, 128 registers without
+// a spill. The 20-step KE gradient (BGK, 128^3) at three, four and five
+// resident blocks: 3.37, 3.25 and 3.52 ms (one cell per thread: 3.59).
+constexpr int kAdjointPairBlocks = 4;
+
 struct AdjointParams {
   double omega, omega_minus;
   double domega_dtau, domega_minus_dtau;  // derivatives of the rates w.r.t. tau
