@@ -45,6 +45,7 @@
 #include "codes.cuh"
 #include "collide.cuh"
 #include "common.cuh"
+#include "pairs.cuh"
 #include "reduce.cuh"
 #include "slab_faces.cuh"
 #include "../../include/lbcube_b200.h"
@@ -105,6 +106,12 @@ struct NativeState {
                                                float, Real (&out)[L::Q]) {
     load_cell<L>(p, g, cell, out);
   }
+  // the pull of two adjacent cells (FP32)
+  template <class L>
+  __device__ __forceinline__ static void pulled_pair(const elem* __restrict__ p, const PairGrid& g,
+                                                     const PairRows& r, float, Real (&out)[2][L::Q]) {
+    gather_pair<L>(p, g, r, out);
+  }
   // the pull on a z-slab, across its faces from halo buffers
   template <class L>
   __device__ __forceinline__ static void pulled_slab(const elem* __restrict__ p, const Grid& g,
@@ -138,6 +145,17 @@ struct ShiftedState {
     });
   }
   template <class L>
+  __device__ __forceinline__ static void pulled_pair(const elem* __restrict__ p, const PairGrid& g,
+                                                     const PairRows& r, float ref, float (&out)[2][L::Q]) {
+    unsigned int w[L::Q];
+    gather_code_pair<L>(p, g, r, w);
+    static_for<L::Q>([&](auto I) {
+      const float2 d = ShiftedStorage<FMT>::template decode_pair<L, LB_I(I)>(w[LB_I(I)], {ref});
+      out[0][LB_I(I)] = d.x;
+      out[1][LB_I(I)] = d.y;
+    });
+  }
+  template <class L>
   __device__ __forceinline__ static void pulled_slab(const elem* __restrict__ p, const Grid& g,
                                                      const Neighbours& n, int x, int y, int z,
                                                      float ref, const elem* __restrict__ halo_lo,
@@ -168,6 +186,50 @@ struct SlabFaces {
   Real* send_lo;
   Real* send_hi;
 };
+
+// Reaction part of adjoint step n at one cell: abar, bbar (ma, mb) and ubar from
+// the pulled A, B (ga, gb), lambda_A, lambda_B at the cell and the advecting
+// velocity; adds the cell's dJ/dk and dJ/domega_c to acc.
+template <class FL, class Real>
+__device__ __forceinline__ void reaction_adjoint_cell(
+    const Real (&ga)[ScalarOf<FL>::type::Q], const Real (&gb)[ScalarOf<FL>::type::Q],
+    const Real (&lA)[ScalarOf<FL>::type::Q], const Real (&lB)[ScalarOf<FL>::type::Q], const Real (&u)[FL::D],
+    const ReactiveParams& rp, Real (&ma)[ScalarOf<FL>::type::Q], Real (&mb)[ScalarOf<FL>::type::Q],
+    Real (&ubar)[FL::D], double (&acc)[2]) {
+  using SL = typename ScalarOf<FL>::type;
+  const Real ca = concentration<SL>(ga), cb = concentration<SL>(gb);
+  double dsa, dsb, dsk;
+  reaction_source_grad<Real>(ca, cb, Real(rp.k), dsa, dsb, dsk);
+  const Real oc = Real(rp.omega_c);
+  const Real inv_cs2 = Real(1.0 / SL::cs2);
+  Real sigma = Real(0), ea = Real(0), eb = Real(0), doc = Real(0);
+  static_for<FL::D>([&](auto D) { ubar[LB_I(D)] = Real(0); });
+  static_for<SL::Q>([&](auto I) {
+    constexpr int i = LB_I(I);
+    constexpr double wd = SL::w[i];
+    const Real w = Real(wd);
+    const Real e = w * (Real(1) + c_dot<SL, i>(u) * inv_cs2);
+    sigma += w * (lA[i] + lB[i]);
+    ea += lA[i] * e;
+    eb += lB[i] * e;
+    doc += lA[i] * (geq<SL, i>(ca, u) - ga[i]) + lB[i] * (geq<SL, i>(cb, u) - gb[i]);
+    const Real s = w * (ca * lA[i] + cb * lB[i]);
+    static_for<FL::D>([&](auto D) {
+      constexpr int c = SL::c[i][LB_I(D)];
+      if constexpr (c > 0) ubar[LB_I(D)] += s;
+      if constexpr (c < 0) ubar[LB_I(D)] -= s;
+    });
+  });
+  static_for<FL::D>([&](auto D) { ubar[LB_I(D)] = ubar[LB_I(D)] * (oc * inv_cs2); });
+  acc[0] += (double)sigma * dsk;
+  acc[1] += (double)doc;
+  const Real sa = Real((double)sigma * dsa), sb = Real((double)sigma * dsb);
+  static_for<SL::Q>([&](auto I) {
+    constexpr int j = LB_I(I);
+    ma[j] = (Real(1) - oc) * lA[j] + oc * ea + sa;
+    mb[j] = (Real(1) - oc) * lB[j] + oc * eb + sb;
+  });
+}
 
 // Reaction part of adjoint step n at every cell x: from the pulled A^n, B^n,
 // lambda_A^{n+1}, lambda_B^{n+1} at x and the advecting velocity u^{n+1}(x)
@@ -210,39 +272,9 @@ __global__ void __launch_bounds__(kThreads)
     }
     load_cell<SL>(la_next, g, cell, lA);
     load_cell<SL>(lb_next, g, cell, lB);
-    const Real ca = concentration<SL>(ga), cb = concentration<SL>(gb);
-    double dsa, dsb, dsk;
-    reaction_source_grad<Real>(ca, cb, Real(rp.k), dsa, dsb, dsk);
-    const Real oc = Real(rp.omega_c);
-    const Real inv_cs2 = Real(1.0 / SL::cs2);
-    Real sigma = Real(0), ea = Real(0), eb = Real(0), doc = Real(0), ubar[FL::D];
-    static_for<FL::D>([&](auto D) { ubar[LB_I(D)] = Real(0); });
-    static_for<SL::Q>([&](auto I) {
-      constexpr int i = LB_I(I);
-      constexpr double wd = SL::w[i];
-      const Real w = Real(wd);
-      const Real e = w * (Real(1) + c_dot<SL, i>(u) * inv_cs2);
-      sigma += w * (lA[i] + lB[i]);
-      ea += lA[i] * e;
-      eb += lB[i] * e;
-      doc += lA[i] * (geq<SL, i>(ca, u) - ga[i]) + lB[i] * (geq<SL, i>(cb, u) - gb[i]);
-      const Real s = w * (ca * lA[i] + cb * lB[i]);
-      static_for<FL::D>([&](auto D) {
-        constexpr int c = SL::c[i][LB_I(D)];
-        if constexpr (c > 0) ubar[LB_I(D)] += s;
-        if constexpr (c < 0) ubar[LB_I(D)] -= s;
-      });
-    });
-    static_for<FL::D>([&](auto D) { ubar_out[plane * LB_I(D) + cell] = ubar[LB_I(D)] * (oc * inv_cs2); });
-    acc[0] = (double)sigma * dsk;
-    acc[1] = (double)doc;
-    const Real sa = Real((double)sigma * dsa), sb = Real((double)sigma * dsb);
-    Real ma[SL::Q], mb[SL::Q];
-    static_for<SL::Q>([&](auto I) {
-      constexpr int j = LB_I(I);
-      ma[j] = (Real(1) - oc) * lA[j] + oc * ea + sa;
-      mb[j] = (Real(1) - oc) * lB[j] + oc * eb + sb;
-    });
+    Real ma[SL::Q], mb[SL::Q], ubar[FL::D];
+    reaction_adjoint_cell<FL, Real>(ga, gb, lA, lB, u, rp, ma, mb, ubar, acc);
+    static_for<FL::D>([&](auto D) { ubar_out[plane * LB_I(D) + cell] = ubar[LB_I(D)]; });
     if constexpr (SLAB) {
       scatter_slab<SL>(la, g, n, x, y, z, ma, faces.send_lo + a_off, faces.send_hi + a_off);
       scatter_slab<SL>(lb, g, n, x, y, z, mb, faces.send_lo + b_off, faces.send_hi + b_off);
@@ -256,6 +288,19 @@ __global__ void __launch_bounds__(kThreads)
     slots[warp_slot(g) * kReactiveSlots + 0] += acc[0];
     slots[warp_slot(g) * kReactiveSlots + 2] += acc[1];
   }
+}
+
+// lambda_f^{n+1}(x, k) += (c_k - u) . ubar(x) / rho.
+template <class FL, class Real>
+__device__ __forceinline__ void add_velocity_adjoint(Real rho, const Real (&u)[FL::D], const Real (&ub)[FL::D],
+                                                     Real (&lv)[FL::Q]) {
+  Real uub = Real(0);
+  static_for<FL::D>([&](auto D) { uub += u[LB_I(D)] * ub[LB_I(D)]; });
+  const Real inv_rho = Real(1) / rho;
+  static_for<FL::Q>([&](auto I) {
+    constexpr int k = LB_I(I);
+    lv[k] += (c_dot<FL, k>(ub) - uub) * inv_rho;
+  });
 }
 
 // Fluid part of adjoint step n: lambda_f^{n+1}(x, k) gains
@@ -283,13 +328,7 @@ __global__ void __launch_bounds__(kThreads, kAdjointBlocks<Real>)
     load_cell<FL>(lf_next, g, cell, lv);
     static_for<FL::D>([&](auto D) { ub[LB_I(D)] = __ldg(ubar_in + plane * LB_I(D) + cell); });
     macro_state<FL>(gv, rho, u);
-    Real uub = Real(0);
-    static_for<FL::D>([&](auto D) { uub += u[LB_I(D)] * ub[LB_I(D)]; });
-    const Real inv_rho = Real(1) / rho;
-    static_for<FL::Q>([&](auto I) {
-      constexpr int k = LB_I(I);
-      lv[k] += (c_dot<FL, k>(ub) - uub) * inv_rho;
-    });
+    add_velocity_adjoint<FL>(rho, u, ub, lv);
     dtau = fluid_adjoint_cell<FL, Real, CT>(gv, lv, rho, u, ap, mu);
     if constexpr (SLAB) scatter_slab<FL>(lf, g, n, x, y, z, mu, faces.send_lo, faces.send_hi);
     else scatter<FL>(lf, g, n, x, y, z, mu);
@@ -297,6 +336,93 @@ __global__ void __launch_bounds__(kThreads, kAdjointBlocks<Real>)
   double v[1] = {dtau};
   warp_sum<1>(v);
   if ((threadIdx.x & 31) == 0) slots[warp_slot(g) * kReactiveSlots + 1] += v[0];
+}
+
+// ---- two FP32 cells per thread (pairs.cuh) -----------------------------------------
+// The same cell functions on pairs, for the planes that neither pull nor scatter
+// across the faces of a slab, from the box on whose one-cell launch no longer fits
+// the SMs at once (native 24^3: 142 -> 168 us per gradient, 64^3 455 -> 442). TRT,
+// FP16 states, 192^3: reaction part 205 -> 185 us (a copy of its 164 B per cell
+// takes 176), fluid part 286 -> 259 (217). Resident blocks of the reaction part: 4
+// (native 128^3 gradient 3.13 ms, 3.20 at 5, 3.28 at 6). Each warp adds to the slots of the first
+// of the one-cell blocks that its block covers.
+constexpr int kReactionPairBlocks = 4;
+
+__device__ __forceinline__ long long pair_warp_slot(const PairGrid& g, int z) {
+  return ((long long)z * g.tiles + (long long)kPairCells * blockIdx.x) * kWarpsPerBlock + (long long)(threadIdx.x >> 5);
+}
+
+template <class FL, class SP>
+__global__ void __launch_bounds__(kThreads, kReactionPairBlocks)
+    reaction_adjoint_pair_kernel(const typename SP::elem* __restrict__ an, const typename SP::elem* __restrict__ bn,
+                                 const float* __restrict__ u_next, const float* __restrict__ la_next,
+                                 const float* __restrict__ lb_next, float* __restrict__ la, float* __restrict__ lb,
+                                 float* __restrict__ ubar_out, PairGrid g, ReactiveParams rp,
+                                 double* __restrict__ slots) {
+  using SL = typename ScalarOf<FL>::type;
+  pdl_enter();
+  int x0, y, z;
+  const bool active = pair_of(g, x0, y, z);
+  double acc[2] = {0.0, 0.0};
+  if (active) {
+    const PairRows r(g, x0, y, z);
+    const int cell = (z * g.ny + y) * g.nx + x0;
+    float u[2][FL::D], ga[2][SL::Q], gb[2][SL::Q], lA[2][SL::Q], lB[2][SL::Q];
+    static_for<FL::D>([&](auto D) {
+      const float2 w = __ldg(reinterpret_cast<const float2*>(u_next + (size_t)g.plane * LB_I(D) + cell));
+      u[0][LB_I(D)] = w.x;
+      u[1][LB_I(D)] = w.y;
+    });
+    SP::template pulled_pair<SL>(an, g, r, rp.c0, ga);
+    SP::template pulled_pair<SL>(bn, g, r, rp.c0, gb);
+    load_pair<SL>(la_next, g, cell, lA);
+    load_pair<SL>(lb_next, g, cell, lB);
+    float ma[2][SL::Q], mb[2][SL::Q], ubar[2][FL::D];
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+      reaction_adjoint_cell<FL, float>(ga[j], gb[j], lA[j], lB[j], u[j], rp, ma[j], mb[j], ubar[j], acc);
+    store_pair(ubar_out, g, cell, ubar);
+    scatter_pair<SL>(la, g, r, ma);
+    scatter_pair<SL>(lb, g, r, mb);
+  }
+  warp_sum<2>(acc);
+  if ((threadIdx.x & 31) == 0) {
+    slots[pair_warp_slot(g, z) * kReactiveSlots + 0] += acc[0];
+    slots[pair_warp_slot(g, z) * kReactiveSlots + 2] += acc[1];
+  }
+}
+
+template <class FL, int CT, class SP>
+__global__ void __launch_bounds__(kThreads, kAdjointPairBlocks)
+    coupled_fluid_adjoint_pair_kernel(const typename SP::elem* __restrict__ fn, const float* __restrict__ lf_next,
+                                      const float* __restrict__ ubar_in, float* __restrict__ lf, PairGrid g,
+                                      AdjointParams ap, float rho0, double* __restrict__ slots) {
+  pdl_enter();
+  int x0, y, z;
+  const bool active = pair_of(g, x0, y, z);
+  double v[1] = {0.0};
+  if (active) {
+    const PairRows r(g, x0, y, z);
+    const int cell = (z * g.ny + y) * g.nx + x0;
+    float gv[2][FL::Q], lv[2][FL::Q], mu[2][FL::Q], ub[2][FL::D];
+    SP::template pulled_pair<FL>(fn, g, r, rho0, gv);
+    load_pair<FL>(lf_next, g, cell, lv);
+    static_for<FL::D>([&](auto D) {
+      const float2 w = __ldg(reinterpret_cast<const float2*>(ubar_in + (size_t)g.plane * LB_I(D) + cell));
+      ub[0][LB_I(D)] = w.x;
+      ub[1][LB_I(D)] = w.y;
+    });
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      float rho, u[FL::D];
+      macro_state<FL>(gv[j], rho, u);
+      add_velocity_adjoint<FL>(rho, u, ub[j], lv[j]);
+      v[0] += fluid_adjoint_cell<FL, float, CT>(gv[j], lv[j], rho, u, ap, mu[j]);
+    }
+    scatter_pair<FL>(lf, g, r, mu);
+  }
+  warp_sum<1>(v);
+  if ((threadIdx.x & 31) == 0) slots[pair_warp_slot(g, z) * kReactiveSlots + 1] += v[0];
 }
 
 // Seeds lambda^N = dJ/d(f^N, A^N, B^N) and writes the block's FP64 share of J.
@@ -419,16 +545,33 @@ __global__ void __launch_bounds__(kThreads)
   static_for<FL::D>([&](auto D) { grad[plane * LB_I(D) + cell] = gr[LB_I(D)]; });
 }
 
+// One adjoint step of planes g.z0 .. g.z0 + planes - 1, no faces of a slab.
 template <class FL, class Real, class SP>
-cudaError_t launch_reactive_adjoint(int collision, const typename SP::elem* fn,
+cudaError_t launch_reactive_adjoint(int collision, int planes, const typename SP::elem* fn,
                                     const typename SP::elem* an, const typename SP::elem* bn,
                                     const Real* u_next, const Real* lf_next, const Real* la_next,
                                     const Real* lb_next, Real* lf, Real* la, Real* lb, Real* ubar,
                                     const Grid& g, const ReactiveParams& rp, double* slots,
                                     cudaStream_t s) {
-  // programmatic dependent launches (both kernels open with pdl_enter)
+  // programmatic dependent launches (the kernels open with pdl_enter)
+  if constexpr (std::is_same_v<Real, float> && FL::Q <= 19) {
+    if (pairs_eligible(g, 12, fn, an, bn, u_next, lf_next, la_next, lb_next, lf, la, lb, ubar)) {
+      const PairGrid pg = make_pair_grid(g, g.z0);
+      const dim3 grid = pair_grid_dims(pg, planes), block(kThreads);
+      const cudaError_t err = launch_pdl(reaction_adjoint_pair_kernel<FL, SP>, grid, block, 0, s, an, bn, u_next,
+                                         la_next, lb_next, la, lb, ubar, pg, rp, slots);
+      if (err != cudaSuccess) return err;
+      auto fluid = [&](auto ct) {
+        return launch_pdl(coupled_fluid_adjoint_pair_kernel<FL, decltype(ct)::value, SP>, grid, block, 0, s, fn,
+                          lf_next, (const float*)ubar, lf, pg, rp.fluid, rp.rho0, slots);
+      };
+      if (collision == kBGK) return fluid(std::integral_constant<int, kBGK>{});
+      if (collision == kTRT) return fluid(std::integral_constant<int, kTRT>{});
+      return fluid(std::integral_constant<int, kMRT>{});
+    }
+  }
   using Faces = SlabFaces<typename SP::elem, Real>;
-  const dim3 grid = grid_dims(g), block(block_dims(g));
+  const dim3 grid((unsigned)g.tiles, (unsigned)planes), block(block_dims(g));
   cudaError_t err = launch_pdl(reaction_adjoint_kernel<FL, Real, SP, false>, grid, block, 0, s, an, bn,
                                u_next, la_next, lb_next, la, lb, ubar, g, rp, slots, Faces{});
   if (err != cudaSuccess) return err;
@@ -645,7 +788,7 @@ cudaError_t reactive_gradient(int collision, int objective, const Real* rho0, co
       const State sn1 = n + 1 == n1 ? ckpt(kk + 1) : seg(n + 1 - n0);  // holds u^{n+1}
       const Adj& ln = lam[(n + 1) % 2];
       const Adj& l = lam[n % 2];
-      err = launch_reactive_adjoint<FL, Real, SP>(collision, sn.f, sn.a, sn.b, sn1.u, ln.f, ln.a,
+      err = launch_reactive_adjoint<FL, Real, SP>(collision, g.nz, sn.f, sn.a, sn.b, sn1.u, ln.f, ln.a,
                                                   ln.b, l.f, l.a, l.b, ubar, g, rp, slots, s);
       if (err != cudaSuccess) return err;
     }
@@ -841,40 +984,30 @@ cudaError_t slab_adjoint_step(int collision, const typename SP::elem* fn,
   const SlabFaces<E, Real> faces{halo_lo, halo_hi, send_lo, send_hi};
   // Planes 1 .. nz-2 pull and scatter only inside the slab: the whole-box
   // kernels (fewer registers than the SLAB forms); planes 0 and nz-1 the SLAB
-  // forms. Every reaction launch precedes the fluid launches (they read its
-  // ubar); slots are indexed by absolute plane.
-  auto ranges = [&](auto each) {
-    if (g.nz >= 3) each(1, g.nz - 2, 1, std::false_type{});
-    each(0, g.nz >= 2 ? 2 : 1, g.nz - 1, std::true_type{});  // both face planes in one launch
-  };
-  ranges([&](int z0, int planes, int zs, auto slab) {
-    constexpr bool SLAB = decltype(slab)::value;
-    Grid gr = g;
-    gr.z0 = z0;
-    gr.zs = zs;
-    dim3 grid = grid_dims(gr);
-    grid.y = (unsigned)planes;
-    launch_pdl(reaction_adjoint_kernel<FL, Real, SP, SLAB>, grid, dim3(block_dims(gr)), 0, s, an, bn,
-               u_next, la_next, lb_next, la, lb, ubar, gr, rp, slots, faces);
-  });
-  ranges([&](int z0, int planes, int zs, auto slab) {
-    constexpr bool SLAB = decltype(slab)::value;
-    Grid gr = g;
-    gr.z0 = z0;
-    gr.zs = zs;
-    dim3 grid = grid_dims(gr);
-    grid.y = (unsigned)planes;
-    const dim3 block(block_dims(gr));
-    if (collision == kBGK)
-      launch_pdl(coupled_fluid_adjoint_kernel<FL, Real, kBGK, SP, SLAB>, grid, block, 0, s, fn, lf_next,
-                 ubar, lf, gr, rp.fluid, rp.rho0, slots, faces);
-    else if (collision == kTRT)
-      launch_pdl(coupled_fluid_adjoint_kernel<FL, Real, kTRT, SP, SLAB>, grid, block, 0, s, fn, lf_next,
-                 ubar, lf, gr, rp.fluid, rp.rho0, slots, faces);
-    else if constexpr (FL::Q != 27)
-      launch_pdl(coupled_fluid_adjoint_kernel<FL, Real, kMRT, SP, SLAB>, grid, block, 0, s, fn, lf_next,
-                 ubar, lf, gr, rp.fluid, rp.rho0, slots, faces);
-  });
+  // forms, both in one launch. A fluid launch reads the ubar of its own cells,
+  // which the reaction launch over the same planes wrote before it; slots are
+  // indexed by absolute plane.
+  if (g.nz >= 3) {
+    Grid gi = g;
+    gi.z0 = 1;
+    const cudaError_t err = launch_reactive_adjoint<FL, Real, SP>(collision, g.nz - 2, fn, an, bn, u_next, lf_next,
+                                                                  la_next, lb_next, lf, la, lb, ubar, gi, rp, slots, s);
+    if (err != cudaSuccess) return err;
+  }
+  Grid gf = g;
+  gf.zs = g.nz - 1;
+  const dim3 grid((unsigned)g.tiles, g.nz >= 2 ? 2 : 1), block(block_dims(g));
+  launch_pdl(reaction_adjoint_kernel<FL, Real, SP, true>, grid, block, 0, s, an, bn, u_next, la_next, lb_next, la,
+             lb, ubar, gf, rp, slots, faces);
+  if (collision == kBGK)
+    launch_pdl(coupled_fluid_adjoint_kernel<FL, Real, kBGK, SP, true>, grid, block, 0, s, fn, lf_next, ubar, lf, gf,
+               rp.fluid, rp.rho0, slots, faces);
+  else if (collision == kTRT)
+    launch_pdl(coupled_fluid_adjoint_kernel<FL, Real, kTRT, SP, true>, grid, block, 0, s, fn, lf_next, ubar, lf, gf,
+               rp.fluid, rp.rho0, slots, faces);
+  else if constexpr (FL::Q != 27)
+    launch_pdl(coupled_fluid_adjoint_kernel<FL, Real, kMRT, SP, true>, grid, block, 0, s, fn, lf_next, ubar, lf, gf,
+               rp.fluid, rp.rho0, slots, faces);
   return cudaGetLastError();
 }
 
