@@ -93,6 +93,7 @@ template <class L, class Real>
 __global__ void __launch_bounds__(kThreads)
     ke_seed_kernel(const Real* __restrict__ f, Real* __restrict__ lam, Grid g,
                    double* __restrict__ ke_slots) {
+  pdl_enter();
   int x, y, z;
   const bool active = cell_of(g, x, y, z);
   double ke = 0.0;
@@ -119,6 +120,7 @@ template <class L, class Real>
 __global__ void __launch_bounds__(kThreads)
     velocity_gradient_kernel(const Real* __restrict__ rho0, const Real* __restrict__ u0,
                              const Real* __restrict__ lam0, Real* __restrict__ grad, Grid g) {
+  pdl_enter();
   int x, y, z;
   if (!cell_of(g, x, y, z)) return;
   const int cell = (z * g.ny + y) * g.nx + x;
@@ -246,8 +248,9 @@ cudaError_t ke_gradient(int collision, const Real* rho0, const Real* u0, const G
     cur = nxt;
   }
   // seed: lambda^N and J from f^N (the last checkpoint written)
-  ke_seed_kernel<L, Real><<<grid_dims(g), block_dims(g), 0, s>>>(cur, lam[steps % 2], g, ke_slots);
-  if ((err = cudaGetLastError()) != cudaSuccess) return err;
+  err = launch_pdl(ke_seed_kernel<L, Real>, grid_dims(g), dim3(block_dims(g)), 0, s, cur, lam[steps % 2], g,
+                   ke_slots);
+  if (err != cudaSuccess) return err;
   if ((err = cudaMemsetAsync(dtau_slots, 0, lay.slots * sizeof(double), s)) != cudaSuccess) return err;
   const AdjointParams ap = make_params<Real>(collision, tau);
   // backward over segments [k*interval, min((k+1)*interval, steps))
@@ -269,11 +272,10 @@ cudaError_t ke_gradient(int collision, const Real* rho0, const Real* u0, const G
       if (err != cudaSuccess) return err;
     }
   }
-  velocity_gradient_kernel<L, Real><<<grid_dims(g), block_dims(g), 0, s>>>(rho0, u0, lam[0], grad_u0, g);
-  if ((err = cudaGetLastError()) != cudaSuccess) return err;
-  sum_slots_kernel<<<1, 1024, 0, s>>>(ke_slots, lay.used, 1, 1.0, out);
-  sum_slots_kernel<<<1, 1024, 0, s>>>(dtau_slots, lay.used, 1, 1.0, out + 1);
-  return cudaGetLastError();
+  err = launch_pdl(velocity_gradient_kernel<L, Real>, grid_dims(g), dim3(block_dims(g)), 0, s, rho0, u0,
+                   (const Real*)lam[0], grad_u0, g);
+  if (err != cudaSuccess) return err;
+  return launch_slot_sums(2, {{{ke_slots, lay.used, 1, 1.0, out}, {dtau_slots, lay.used, 1, 1.0, out + 1}}}, s);
 }
 
 template <class Real>

@@ -439,6 +439,7 @@ __global__ void __launch_bounds__(kThreads)
                          Real* __restrict__ la, Real* __restrict__ lb, Grid g, float c0,
                          double inv_n, double* __restrict__ j_slots) {
   using SL = typename ScalarOf<FL>::type;
+  pdl_enter();
   int x, y, z;
   const bool active = cell_of(g, x, y, z);
   double jpart = 0.0;
@@ -481,6 +482,7 @@ __global__ void __launch_bounds__(kThreads)
     scalar_init_gradient_kernel(const Real* __restrict__ u0, const Real* __restrict__ lam0,
                                 Real direct, Real* __restrict__ grad, Grid g) {
   using SL = typename ScalarOf<FL>::type;
+  pdl_enter();
   int x, y, z;
   if (!cell_of(g, x, y, z)) return;
   const int cell = (z * g.ny + y) * g.nx + x;
@@ -508,6 +510,7 @@ __global__ void __launch_bounds__(kThreads)
                                       const Real* __restrict__ lf, const Real* __restrict__ la,
                                       const Real* __restrict__ lb, Real* __restrict__ grad, Grid g) {
   using SL = typename ScalarOf<FL>::type;
+  pdl_enter();
   int x, y, z;
   if (!cell_of(g, x, y, z)) return;
   const int cell = (z * g.ny + y) * g.nx + x;
@@ -737,6 +740,7 @@ cudaError_t reactive_gradient(int collision, int objective, const Real* rho0, co
   }
 
   // seed lambda^N and J
+  const dim3 grid = grid_dims(g), block(block_dims(g));
   const Adj& lN = lam[steps % 2];
   if (objective == LBM_OBJECTIVE_SEGREGATION) {
     const Real* fa = reinterpret_cast<const Real*>(cur.a);
@@ -755,13 +759,11 @@ cudaError_t reactive_gradient(int collision, int objective, const Real* rho0, co
                                                 (size_t)lay.blocks * kStatSums * sizeof(double),
                                                 stats, s);
     if (err != cudaSuccess) return err;
-    reactive_seed_kernel<FL, Real, LBM_OBJECTIVE_SEGREGATION, SP>
-        <<<grid_dims(g), block_dims(g), 0, s>>>(cur.a, cur.b, a0, stats, lN.f, lN.a, lN.b, g, c0,
-                                                1.0 / (double)g.plane, j_slots);
+    launch_pdl(reactive_seed_kernel<FL, Real, LBM_OBJECTIVE_SEGREGATION, SP>, grid, block, 0, s, cur.a, cur.b, a0,
+               stats, lN.f, lN.a, lN.b, g, c0, 1.0 / (double)g.plane, j_slots);
   } else {
-    reactive_seed_kernel<FL, Real, LBM_OBJECTIVE_MEAN_PRODUCT, SP>
-        <<<grid_dims(g), block_dims(g), 0, s>>>(cur.a, cur.b, a0, stats, lN.f, lN.a, lN.b, g, c0,
-                                                1.0 / (double)g.plane, j_slots);
+    launch_pdl(reactive_seed_kernel<FL, Real, LBM_OBJECTIVE_MEAN_PRODUCT, SP>, grid, block, 0, s, cur.a, cur.b, a0,
+               stats, lN.f, lN.a, lN.b, g, c0, 1.0 / (double)g.plane, j_slots);
   }
   if ((err = cudaGetLastError()) != cudaSuccess) return err;
   if ((err = cudaMemsetAsync(slots, 0,
@@ -797,27 +799,22 @@ cudaError_t reactive_gradient(int collision, int objective, const Real* rho0, co
   // results: J, dJ/dk, dJ/dtau, dJ/dtau_c; dJ/dA0 (and dJ/dB0, dJ/du0). For
   // 16-bit states the encoding of the initial state counts as the identity.
   const Real direct_a = objective == LBM_OBJECTIVE_MEAN_PRODUCT ? Real(1.0 / (double)g.plane) : Real(0);
-  scalar_init_gradient_kernel<FL, Real><<<grid_dims(g), block_dims(g), 0, s>>>(u0, lam[0].a, direct_a,
-                                                                          grad_a0, g);
+  launch_pdl(scalar_init_gradient_kernel<FL, Real>, grid, block, 0, s, u0, lam[0].a, direct_a, grad_a0, g);
   if (grad_b0 != nullptr)
-    scalar_init_gradient_kernel<FL, Real><<<grid_dims(g), block_dims(g), 0, s>>>(u0, lam[0].b, Real(0),
-                                                                            grad_b0, g);
+    launch_pdl(scalar_init_gradient_kernel<FL, Real>, grid, block, 0, s, u0, lam[0].b, Real(0), grad_b0, g);
   if (grad_u0 != nullptr)
-    reactive_velocity_gradient_kernel<FL, Real><<<grid_dims(g), block_dims(g), 0, s>>>(
-        rho0, u0, a0, b0, lam[0].f, lam[0].a, lam[0].b, grad_u0, g);
-  if (objective == LBM_OBJECTIVE_SEGREGATION) {
-    if ((err = cudaMemcpyAsync(out, stats + 5, sizeof(double), cudaMemcpyDeviceToDevice, s)) !=
-        cudaSuccess)
-      return err;
-  } else {
-    sum_slots_kernel<<<1, 1024, 0, s>>>(j_slots, g.launched(), 1, 1.0 / (double)g.plane, out);
-  }
+    launch_pdl(reactive_velocity_gradient_kernel<FL, Real>, grid, block, 0, s, rho0, u0, a0, b0, lam[0].f,
+               lam[0].a, lam[0].b, grad_u0, g);
+  if ((err = cudaGetLastError()) != cudaSuccess) return err;
   const long long nslots = g.launched() * kWarpsPerBlock;
-  sum_slots_kernel<<<1, 1024, 0, s>>>(slots + 0, nslots, kReactiveSlots, 1.0, out + 1);
-  sum_slots_kernel<<<1, 1024, 0, s>>>(slots + 1, nslots, kReactiveSlots, 1.0, out + 2);
-  sum_slots_kernel<<<1, 1024, 0, s>>>(slots + 2, nslots, kReactiveSlots, -omega_c * omega_c,
-                                      out + 3);
-  return cudaGetLastError();
+  SlotSums sums{{{slots + 0, nslots, kReactiveSlots, 1.0, out + 1},
+                 {slots + 1, nslots, kReactiveSlots, 1.0, out + 2},
+                 {slots + 2, nslots, kReactiveSlots, -omega_c * omega_c, out + 3},
+                 {j_slots, g.launched(), 1, 1.0 / (double)g.plane, out}}};
+  if (objective != LBM_OBJECTIVE_SEGREGATION) return launch_slot_sums(4, sums, s);
+  if ((err = cudaMemcpyAsync(out, stats + 5, sizeof(double), cudaMemcpyDeviceToDevice, s)) != cudaSuccess)
+    return err;
+  return launch_slot_sums(3, sums, s);
 }
 
 inline int scalar_q(int fluid_lattice) { return fluid_lattice == kD2Q9 ? 5 : 7; }
@@ -1248,11 +1245,11 @@ extern "C" int lbm_reactive_slab_seed_async(int fluid_lattice, int precision, in
     using SP = SlabState<R, decltype(f)::value>;
     using E = typename SP::elem;
     if (objective == LBM_OBJECTIVE_SEGREGATION)
-      reactive_seed_kernel<FL, R, LBM_OBJECTIVE_SEGREGATION, SP><<<grid_dims(g), block_dims(g), 0, s>>>(
+      launch_pdl(reactive_seed_kernel<FL, R, LBM_OBJECTIVE_SEGREGATION, SP>, grid_dims(g), dim3(block_dims(g)), 0, s,
           (const E*)a_final, (const E*)b_final, (const R*)a0, diagnostics, (R*)lambda_fluid,
           (R*)lambda_a, (R*)lambda_b, g, c0, inv_n, objective_partials);
     else
-      reactive_seed_kernel<FL, R, LBM_OBJECTIVE_MEAN_PRODUCT, SP><<<grid_dims(g), block_dims(g), 0, s>>>(
+      launch_pdl(reactive_seed_kernel<FL, R, LBM_OBJECTIVE_MEAN_PRODUCT, SP>, grid_dims(g), dim3(block_dims(g)), 0, s,
           (const E*)a_final, (const E*)b_final, (const R*)a0, diagnostics, (R*)lambda_fluid,
           (R*)lambda_a, (R*)lambda_b, g, c0, inv_n, objective_partials);
     return (int)cudaGetLastError();
@@ -1281,13 +1278,13 @@ extern "C" int lbm_reactive_slab_init_gradients_async(
     using FL = decltype(fl);
     using R = decltype(r);
     const R direct = objective == LBM_OBJECTIVE_MEAN_PRODUCT ? R(1.0 / total_cells) : R(0);
-    scalar_init_gradient_kernel<FL, R><<<grid_dims(g), block_dims(g), 0, s>>>(
+    launch_pdl(scalar_init_gradient_kernel<FL, R>, grid_dims(g), dim3(block_dims(g)), 0, s,
         (const R*)u0, (const R*)lambda_a, direct, (R*)grad_a0, g);
     if (grad_b0 != nullptr)
-      scalar_init_gradient_kernel<FL, R><<<grid_dims(g), block_dims(g), 0, s>>>(
+      launch_pdl(scalar_init_gradient_kernel<FL, R>, grid_dims(g), dim3(block_dims(g)), 0, s,
           (const R*)u0, (const R*)lambda_b, R(0), (R*)grad_b0, g);
     if (grad_u0 != nullptr)
-      reactive_velocity_gradient_kernel<FL, R><<<grid_dims(g), block_dims(g), 0, s>>>(
+      launch_pdl(reactive_velocity_gradient_kernel<FL, R>, grid_dims(g), dim3(block_dims(g)), 0, s,
           (const R*)rho0, (const R*)u0, (const R*)a0, (const R*)b0, (const R*)lambda_fluid,
           (const R*)lambda_a, (const R*)lambda_b, (R*)grad_u0, g);
     return (int)cudaGetLastError();
@@ -1307,10 +1304,9 @@ extern "C" int lbm_reactive_slab_sums_async(int fluid_lattice, size_t x_extent, 
     return (int)cudaErrorInvalidValue;
   const cudaStream_t s = as_stream(stream);
   const long long nslots = g.launched() * kWarpsPerBlock;
-  sum_slots_kernel<<<1, 1024, 0, s>>>(objective_partials, g.launched(), 1, 1.0, sums);
-  for (int k = 0; k < kReactiveSlots; ++k)
-    sum_slots_kernel<<<1, 1024, 0, s>>>(slots + k, nslots, kReactiveSlots, 1.0, sums + 1 + k);
-  return (int)cudaGetLastError();
+  SlotSums all{{{objective_partials, g.launched(), 1, 1.0, sums}}};
+  for (int k = 0; k < kReactiveSlots; ++k) all.sum[1 + k] = {slots + k, nslots, kReactiveSlots, 1.0, sums + 1 + k};
+  return (int)launch_slot_sums(1 + kReactiveSlots, all, s);
 }
 
 extern "C" int lbm_reactive_slab_result_async(int precision, int objective, const double* sums,

@@ -155,6 +155,7 @@ template <class L, int FMT, class Real, bool ENCODE>
 __global__ void __launch_bounds__(256)
     convert_kernel(const void* __restrict__ in, void* __restrict__ out, long long plane,
                    float rho0) {
+  pdl_enter();
   using S = ShiftedStorage<FMT>;
   const typename S::Params p{rho0};
   const int i = (int)blockIdx.y;
@@ -182,6 +183,7 @@ template <class L, int FMT, bool ENCODE>
 __global__ void __launch_bounds__(256)
     convert4_kernel(const void* __restrict__ in, void* __restrict__ out, long long plane,
                     float rho0) {
+  pdl_enter();
   using S = ShiftedStorage<FMT>;
   const typename S::Params p{rho0};
   const int i = (int)blockIdx.y;
@@ -229,15 +231,12 @@ cudaError_t launch_convert(int precision, const void* in, void* out, size_t nx, 
       (uintptr_t)out % 16 == 0) {
     const dim3 grid4((unsigned)std::min<long long>((g.plane / 4 + 255) / 256, 148LL * 8),
                      (unsigned)L::Q, 1);
-    convert4_kernel<L, FMT, ENCODE><<<grid4, 256, 0, s>>>(in, out, g.plane, rho0);
-    return cudaGetLastError();
+    return launch_pdl(convert4_kernel<L, FMT, ENCODE>, grid4, dim3(256), 0, s, in, out, g.plane, rho0);
   }
   const dim3 grid((unsigned)std::min<long long>((g.plane + 255) / 256, 148LL * 8), (unsigned)L::Q, 1);
   if (precision == LBM_FLOAT)
-    convert_kernel<L, FMT, float, ENCODE><<<grid, 256, 0, s>>>(in, out, g.plane, rho0);
-  else
-    convert_kernel<L, FMT, double, ENCODE><<<grid, 256, 0, s>>>(in, out, g.plane, rho0);
-  return cudaGetLastError();
+    return launch_pdl(convert_kernel<L, FMT, float, ENCODE>, grid, dim3(256), 0, s, in, out, g.plane, rho0);
+  return launch_pdl(convert_kernel<L, FMT, double, ENCODE>, grid, dim3(256), 0, s, in, out, g.plane, rho0);
 }
 
 template <int FMT, bool ENCODE>
