@@ -453,7 +453,7 @@ __device__ __forceinline__ void moments_d3q27(const Real (&f)[27], Real (&m)[27]
   m[2] = raw[t27(0, 1, 0)];
   m[3] = raw[t27(0, 0, 1)];
   m[4] = r200 + r020 + r002;
-  m[5] = Real{2} * r200 - r020 - r002;
+  m[5] = r200 + r200 - r020 - r002;  // 2 r200 exactly
   m[6] = r020 - r002;
   m[7] = raw[t27(1, 1, 0)];
   m[8] = raw[t27(0, 1, 1)];
@@ -532,6 +532,8 @@ struct SafeDividends<double> {
 // The reference's form, IEEE divisions and every term. Out of line, so that
 // the rare cells that need it keep its divisions out of the kernel's
 // instruction stream.
+__device__ __forceinline__ float triple(float x) { return 3.0f * x; }
+__device__ __forceinline__ double triple(double x) { return 3.0 * x; }
 template <class Real>
 __device__ __forceinline__ void moments_to_raw27(const Real (&m)[27], Real (&raw)[27]) {
   raw[t27(0, 0, 0)] = m[0];
@@ -539,8 +541,9 @@ __device__ __forceinline__ void moments_to_raw27(const Real (&m)[27], Real (&raw
   raw[t27(0, 1, 0)] = m[2];
   raw[t27(0, 0, 1)] = m[3];
   raw[t27(2, 0, 0)] = m[4] + m[5];  // times 3, 6 and 6: divided by the callers
-  raw[t27(0, 2, 0)] = Real{2} * m[4] - m[5] + Real{3} * m[6];
-  raw[t27(0, 0, 2)] = Real{2} * m[4] - m[5] - Real{3} * m[6];
+  const Real twice = m[4] + m[4] - m[5], thrice = triple(m[6]);
+  raw[t27(0, 2, 0)] = twice + thrice;
+  raw[t27(0, 0, 2)] = twice - thrice;
   raw[t27(1, 1, 0)] = m[7];
   raw[t27(0, 1, 1)] = m[8];
   raw[t27(1, 0, 1)] = m[9];
@@ -667,15 +670,16 @@ __device__ __forceinline__ void equilibrium_d3q27(Real rho, const Real (&u)[3], 
 }
 
 // Moment relaxation with MrtRelaxationRates_D3Q27 (lattice_mrt.hpp:161-204).
+template <int i, class Real>
+__device__ __forceinline__ Real rate_d3q27(Real omega) {
+  const Real s_b = Real(1.19), s_e = Real(1.1), s_eps = Real(1.2), s_q = Real(1.2);
+  return i == 4 ? s_b : (i <= 9 ? omega : (i <= 15 ? s_e : (i == 16 ? s_eps : s_q)));
+}
 template <class Real>
 __device__ __forceinline__ void relax_d3q27(Real (&m)[27], const Real (&eq)[27], Real omega) {
-  const Real s_b = Real(1.19), s_e = Real(1.1), s_eps = Real(1.2), s_q = Real(1.2);
   static_for<27>([&](auto I) {
     constexpr int i = LB_I(I);
-    if constexpr (i >= 4) {
-      const Real s = i == 4 ? s_b : (i <= 9 ? omega : (i <= 15 ? s_e : (i == 16 ? s_eps : s_q)));
-      m[i] -= s * (m[i] - eq[i]);
-    }
+    if constexpr (i >= 4) m[i] -= rate_d3q27<i>(omega) * (m[i] - eq[i]);
   });
 }
 

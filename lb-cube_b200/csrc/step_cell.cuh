@@ -15,6 +15,7 @@
 #include "collide.cuh"
 #include "common.cuh"
 #include "diag.cuh"
+#include "packed.cuh"
 #include "pairs.cuh"
 
 namespace lbcube {
@@ -133,19 +134,20 @@ __global__ void __launch_bounds__(kThreads)
 // (0: the compiler's choice): D3Q19 7 (72 registers; TRT 180 x 170 x 190 140 us
 // against 143 at 6 and 142 at 8; MRT 151, 159 and 154), RLBM, D2Q9 and D3Q27 the
 // compiler's (D3Q27 BGK 72 x 70 x 68 9.8 us against 11.0 at 4).
+// D3Q27 MRT, in packed arithmetic, 4 (128 registers; 128^3 in a loop of its own
+// 83.6 us against 92 at 3 and 86 at 5, which spills).
 template <class L, int CT>
-constexpr int kPairBlocks = L::Q == 19 && CT != kRLBM ? 7 : 0;
-// Not the D3Q27 MRT, whose 54 populations and as many moments leave too few
-// warps (72 x 70 x 68 16.4 -> 18.6 us).
+constexpr int kPairBlocks = L::Q == 27 && CT == kMRT ? 4 : L::Q == 19 && CT != kRLBM ? 7 : 0;
 template <class L, class Real, int CT>
-constexpr bool kUsePairs = sizeof(Real) == 4 && !(L::Q == 27 && CT == kMRT);
+constexpr bool kUsePairs = sizeof(Real) == 4;
 // From how many one-cell blocks per SM on (pairs_eligible): what the SMs hold
 // at once. D3Q19 12: MRT 56^3 (9.3 blocks per SM) 6.6 -> 7.1 us, 64^3 (13.8) 7.7 ->
 // 6.8. D2Q9 16: MRT 512^2 (13.8) 4.2 -> 5.2, 600^2 (19) 5.1 -> 5.0, 724^2 6.5 -> 5.8.
 // D3Q27 likewise: BGK 64^3 (13.8) level, 72^3 (19.7) 11.5 -> 10.4; its RLBM later:
-// 72^3 18.0 -> 18.4, 88^3 (36) 36.6 -> 33.7.
+// 72^3 18.0 -> 18.4, 88^3 (36) 36.6 -> 33.7; and its MRT: 60 x 62 x 64 (13.4) 11.9 ->
+// 12.4, 72^3 17.7 -> 18.0, 88 x 90 x 86 (35) 30.8 -> 29.4.
 template <class L, int CT>
-constexpr int kPairFrom = L::Q == 19 ? 12 : L::Q == 27 && CT == kRLBM ? 30 : 16;
+constexpr int kPairFrom = L::Q == 19 ? 12 : L::Q == 27 && (CT == kRLBM || CT == kMRT) ? 30 : 16;
 
 template <class L, int CT, bool DIAG, bool FIRST>
 __global__ void __launch_bounds__(kThreads, kPairBlocks<L, CT>)
@@ -158,8 +160,7 @@ __global__ void __launch_bounds__(kThreads, kPairBlocks<L, CT>)
   if (active) {
     float f[2][L::Q];
     gather_pair<L, FIRST>(cur, g, PairRows(g, x0, y, z), f);
-#pragma unroll
-    for (int j = 0; j < 2; ++j) collide<L, float, CT>(f[j], omega, omega_minus);
+    collide_pair<L, CT>(f, omega, omega_minus);
     store_pair(nxt, g, (z * g.ny + y) * g.nx + x0, f);
     if constexpr (DIAG) {
 #pragma unroll

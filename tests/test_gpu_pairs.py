@@ -26,7 +26,8 @@ pytestmark = pytest.mark.gpu
 REALS = {"float": np.float32, "double": np.float64}
 FLUID = [("D3Q19", "float", op, (66, 62, 60)) for op in ("BGK", "TRT", "MRT", "RLBM")]
 FLUID += [("D2Q9", "float", op, (602, 598, 1)) for op in ("BGK", "TRT", "MRT", "RLBM")]
-FLUID += [("D3Q27", "float", op, (70, 68, 66)) for op in ("BGK", "TRT")] + [("D3Q27", "float", "RLBM", (90, 86, 84))]
+FLUID += [("D3Q27", "float", op, (70, 68, 66)) for op in ("BGK", "TRT")]
+FLUID += [("D3Q27", "float", op, (90, 86, 84)) for op in ("MRT", "RLBM")]
 # buffers just above the L2: evict-first loads, pairs, single cells, plane pointers, FP64
 FLUID += [("D3Q19", "float", "TRT", (98, 96, 94)), ("D3Q19", "float", "BGK", (97, 95, 95)),
           ("D3Q19", "float", "MRT", (97, 95, 95)), ("D3Q27", "float", "MRT", (82, 84, 84)),
@@ -42,6 +43,31 @@ def test_step_bitwise(engine, dev, lat, real, op, dims):
     engine.check(engine.launch_step_gpu(lat, real, op, cur, nxt, *dims, 1 / 0.6))
     torch.cuda.synchronize()
     assert U.same_bits(nxt.cpu().numpy(), O.step(f0, lat, op, *dims, 1 / 0.6, steps=1))
+
+
+@pytest.mark.parametrize("shift", [0, 1])
+def test_packed_d3q27_mrt_mixed_cells(engine, dev, shift):
+    """Cells inside and outside the bounds of the fast path in one pair: ordinary
+    cells next to tiny (subnormal moments, dividends around 2^-123), huge, zero,
+    negative-zero and non-finite ones, whose populations reach their neighbours
+    as the step pulls."""
+    dims = (90, 86, 84)
+    n = dims[0] * dims[1] * dims[2]
+    f0 = U.random_state("D3Q27", *dims, np.float64, seed=21, neq=2e-2)
+    kind = (np.arange(n) + shift) % 97
+    for k, scale in ((3, 2.0 ** -104), (11, 2.0 ** -110), (19, 2.0 ** -116), (27, 2.0 ** -122), (35, 2.0 ** -140),
+                     (43, 2.0 ** 61), (51, 2.0 ** 100), (59, 0.0), (67, -0.0)):
+        f0[:, kind == k] *= scale
+    f0 = f0.astype(np.float32)
+    f0[4, np.flatnonzero(kind == 75)[::50]] = np.inf
+    f0[9, np.flatnonzero(kind == 83)[::50]] = np.nan
+    cur = torch.from_numpy(f0).to(dev)
+    nxt = torch.empty_like(cur)
+    engine.check(engine.launch_step_gpu("D3Q27", "float", "MRT", cur, nxt, *dims, 1 / 0.6))
+    torch.cuda.synchronize()
+    with np.errstate(all="ignore"):
+        want = O.step(f0, "D3Q27", "MRT", *dims, 1 / 0.6, steps=1)
+    assert U.same_bits(nxt.cpu().numpy(), want)
 
 
 @pytest.mark.parametrize("lat,op,dims", [("D3Q19", "TRT", (66, 62, 60)), ("D2Q9", "MRT", (602, 598, 1)),
