@@ -248,14 +248,16 @@ __global__ void __launch_bounds__(kThreads, kCoupledCodeBlocks)
 }
 
 // Whether the four-cell kernel steps a range of planes: whole words per row,
-// word-aligned buffers, and a 16-byte aligned velocity output. D3Q27 keeps the
-// one-cell kernel (its 27 words alone fill the register budget).
-template <class FL>
+// word-aligned buffers, a 16-byte aligned velocity output, and a box that
+// coupled_codes_rule takes. D3Q27 keeps the one-cell kernel (its 27 words alone
+// fill the register budget).
+template <class FL, int FMT, int CT, bool STATS, bool UOUT>
 inline bool coupled_codes_eligible(const Grid& g, std::initializer_list<const void*> codes, const float* u_out) {
   if (FL::Q > 19 || g.nx % kCodeCells != 0 || (uintptr_t)u_out % 16 != 0) return false;
   for (const void* p : codes)
     if ((uintptr_t)p % 8 != 0) return false;
-  return true;
+  const int resident = resident_blocks<fluid_reaction_shifted_kernel<FL, FMT, CT, STATS, UOUT, false>>();
+  return several_cells_pay(g.nx, g.ny, g.nz, kCodeCells, kThreads, coupled_codes_rule<FL, FMT>(resident));
 }
 
 // Planes [z0, z0 + planes) without the faces of a slab, by whichever kernel applies.
@@ -267,7 +269,7 @@ cudaError_t launch_coupled_planes(const unsigned short* cf, unsigned short* nf, 
                                   cudaStream_t s) {
   // programmatic dependent launches (the kernels open with pdl_enter)
   if constexpr (FL::Q <= 19) {
-    if (coupled_codes_eligible<FL>(g, {cf, nf, ca, na, cb, nb}, u_out)) {
+    if (coupled_codes_eligible<FL, FMT, CT, STATS, UOUT>(g, {cf, nf, ca, na, cb, nb}, u_out)) {
       const CodeGrid cg = make_code_grid(g, z0);
       const unsigned words = (unsigned)(cg.words * g.ny);
       return launch_pdl(fluid_reaction_codes_kernel<FL, FMT, CT, STATS, UOUT>,

@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <climits>
 #include <cstddef>
 #include <cstdint>
@@ -16,6 +17,7 @@ namespace lbcube {
 // Most threads per block. In the one-cell-per-thread kernels a block covers
 // kThreads consecutive cells of one z plane.
 constexpr int kThreads = 128;
+constexpr int kSMs = 148;
 
 // Division of n < 2^31 by an invariant d < 2^31 as one high product and a
 // shift: mul = ceil(2^(31 + l) / d) with l = ceil(log2 d), so that mul < 2^32 and
@@ -141,6 +143,45 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
+
+// When a launch of several adjacent cells per thread beats one cell per thread. In
+// `blocks per SM` of kThreads-thread blocks: `one` of the one-cell launch, `many` of
+// the other.
+// * from: above this many one-cell blocks per SM, about what the SMs hold at once or
+//   more; below it the one-cell launch's many threads hide more latency than the
+//   saved instructions are worth.
+// * lo, hi: also where one > lo and many <= hi. The next launch of a stream waits
+//   on the SMs while one runs (pdl_enter), so a launch goes without a second wave
+//   up to half of the resident blocks: between the halves of the two kernels
+//   (lo, hi) only the one-cell launch takes the second wave.
+// * unit: a plane's threads fill whole blocks (kThreads) where idle warps wait at a
+//   barrier or hold a large block's registers, whole warps (32) elsewhere; a plane
+//   that this pads by over 15 % more than the one-cell launch keeps one cell per thread.
+struct CellRule {
+  double from, lo = 0, hi = 0;
+};
+inline bool several_cells_pay(int nx, int ny, int nz, int cells, int unit, const CellRule& r) {
+  const long long plane = (long long)nx * ny, threads = plane / cells;
+  auto up = [](long long n, long long to) { return (n + to - 1) / to; };
+  const double one = (double)up(plane, kThreads) * nz / kSMs, many = (double)up(threads, kThreads) * nz / kSMs;
+  if (one > r.lo && many <= r.hi) return true;
+  return one > r.from && 20 * up(threads, unit) * cells <= 23 * up(plane, unit);
+}
+
+// How many blocks of kThreads an SM holds of a kernel: a property of the compiled
+// kernel, asked for until it is known (0: it cannot be told).
+template <auto* kernel>
+inline int resident_blocks() {
+  static std::atomic<int> known{0};
+  int n = known.load(std::memory_order_relaxed);
+  if (n != 0) return n;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, kThreads, 0) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return 0;
+  }
+  known.store(n, std::memory_order_relaxed);
+  return n;
 }
 
 inline dim3 grid_dims(const Grid& g) { return dim3((unsigned)g.tiles, (unsigned)g.nz, 1); }

@@ -59,6 +59,24 @@ inline CodeGrid make_code_grid(const Grid& g, int z0 = 0, int z_step = 1) {
   return c;
 }
 
+// When the coupled fluid + A + B -> C step on 16-bit codes takes four cells per
+// thread, `resident` being how many blocks of its one-cell kernel an SM holds. The
+// four-cell kernel is straight-line code for four collisions and reactions at 5
+// resident blocks: 4.2 us for the smallest box, where one cell per thread takes 2.
+// One step in us, one cell -> four, at one-cell blocks per SM: D3Q19 FP16 TRT 32^3
+// (1.7) 2.6 -> 4.6, 48^3 (5.8) 5.7 -> 5.0, 64 x 64 x 32 (6.9) 5.7 -> 5.1, 56^3 (9.5) 6.4 ->
+// 8.0, 64^3 (13.8) 8.4 -> 8.1, 80^3 (27) 15.4 -> 11.7; E3M12 64^3 12.2 -> 14.2, 76^3 (23.6)
+// 20.0 -> 20.3, 80^3 22.9 -> 22.4; Q15 MRT 64^3 9.9 -> 10.6, 80^3 17.7 -> 16.6. D2Q9 FP16
+// TRT 320^2 (5.4) 3.25 -> 3.37, 352^2 (6.5) 3.7 -> 3.4, 512^2 6.4 -> 5.7; E3M12 512^2 8.3 ->
+// 9.2, 704^2 (26) 13.9 -> 12.5; Q15 640^2 (21.6) 9.4 -> 9.7, 704^2 11.1 -> 10.6.
+template <class FL, int FMT>
+inline CellRule coupled_codes_rule(int resident) {
+  constexpr bool kFloats = FMT == kF16S || FMT == kBF16S;
+  constexpr double from = FL::Q == 9 ? (kFloats ? 6 : 24) : (kFloats ? 13 : 26);
+  constexpr double hi = kFloats ? 2.5 : 2;  // half of 5; the integer codecs lose the wave at 52^3 (2.1)
+  return resident <= 0 ? CellRule{from} : CellRule{from, resident / 2.0 < 4 ? 4 : resident / 2.0, hi};
+}
+
 inline bool codes_eligible(const Grid& g, const void* a, const void* b) {
   return g.nx % kCodeCells == 0 && (uintptr_t)a % 8 == 0 && (uintptr_t)b % 8 == 0;
 }

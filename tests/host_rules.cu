@@ -1,0 +1,40 @@
+// Test helper: answers questions about the host side of the kernels' launch rules,
+// one per line of standard input, from the engine's own headers.
+//   div n d            n / d through FastDiv
+//   coupled L FMT RESIDENT nx ny nz    1 if the 16-bit coupled step takes four cells per thread
+// (L: 9 or 19; FMT: 0 FP16, 1 BF16, 2 E3M12, 3 Q15; RESIDENT: blocks of its one-cell kernel per SM)
+#include <cstdio>
+#include <cstring>
+
+#include "../lb-cube_b200/csrc/stream_codes.cuh"
+
+using namespace lbcube;
+
+template <class L>
+int coupled_of(int fmt, int resident, const Grid& g) {
+  const CellRule r = fmt == kF16S    ? coupled_codes_rule<L, kF16S>(resident)
+                     : fmt == kBF16S ? coupled_codes_rule<L, kBF16S>(resident)
+                                     : coupled_codes_rule<L, kQ15S>(resident);
+  return g.nx % kCodeCells == 0 && several_cells_pay(g.nx, g.ny, g.nz, kCodeCells, kThreads, r);
+}
+
+int main() {
+  char what[16];
+  while (scanf("%15s", what) == 1) {
+    if (strcmp(what, "div") == 0) {
+      unsigned n, d;
+      if (scanf("%u %u", &n, &d) != 2) return 2;
+      printf("%u\n", FastDiv(d)(n));
+      continue;
+    }
+    int a[3];
+    size_t n[3];
+    for (int& v : a)
+      if (scanf("%d", &v) != 1) return 2;
+    if (scanf("%zu %zu %zu", &n[0], &n[1], &n[2]) != 3) return 2;
+    Grid g{};
+    if (validate_domain(false, 1, 1, 1, n[2] == 1 ? 2 : 3, n[0], n[1], n[2], g) != cudaSuccess) return 3;
+    printf("%d\n", a[0] == 9 ? coupled_of<D2Q9>(a[1], a[2], g) : coupled_of<D3Q19>(a[1], a[2], g));
+  }
+  return 0;
+}

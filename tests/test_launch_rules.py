@@ -1,0 +1,70 @@
+"""CPU: the host side of the kernels' launch rules (csrc/common.cuh and the rules of
+the several-cell kernels), compiled from the engine's own headers
+(host_rules.cu) and asked on the host.
+
+* FastDiv equals floor division.
+* Which boxes take several cells per thread. Each expectation is the faster
+  kernel of the two as timed on a B200 (the figures stand beside the rules)."""
+import os
+import random
+import shutil
+import subprocess
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+NVCC = os.environ.get("NVCC", shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc")
+F16, BF16, E3M12, Q15 = range(4)
+
+
+@pytest.fixture(scope="module")
+def ask(tmp_path_factory):
+    if not os.path.exists(NVCC):
+        pytest.skip("no nvcc")
+    exe = str(tmp_path_factory.mktemp("rules") / "host_rules")
+    subprocess.run([NVCC, "-std=c++17", "-O1", "-gencode", "arch=compute_100a,code=sm_100a", "-o", exe,
+                    os.path.join(HERE, "host_rules.cu")], check=True)
+
+    def run(lines):
+        out = subprocess.run([exe], input="\n".join(lines) + "\n", check=True, capture_output=True, text=True).stdout
+        rows = [[int(v) for v in line.split()] for line in out.splitlines()]
+        assert len(rows) == len(lines)
+        return rows
+
+    return run
+
+
+def test_fast_div(ask):
+    rng = random.Random(6)
+    top = 2 ** 31 - 1
+    ds = {1, 2, 3, 5, 7, 127, 128, 129, 1024, top, top - 1}
+    ds |= {(1 << k) + e for k in range(1, 31) for e in (-1, 0, 1)} | {int(2 ** rng.uniform(0, 31)) for _ in range(200)}
+    pairs = []
+    for d in sorted(d for d in ds if 1 <= d <= top):
+        ns = {0, 1, d - 1, d, min(top, 2 * d - 1), top, top // d * d, max(0, top // d * d - 1)}
+        ns |= {min(top, rng.randint(0, top // d) * d + e) for _ in range(10) for e in (0, d - 1)}
+        pairs += [(n, d) for n in sorted(ns)]
+    for (n, d), (q,) in zip(pairs, ask([f"div {n} {d}" for n, d in pairs])):
+        assert q == n // d, (n, d)
+
+
+COUPLED = [
+    # lattice, format, resident one-cell blocks per SM, box, four cells per thread
+    (19, F16, 9, (8, 8, 8), 0), (19, F16, 9, (32, 32, 32), 0), (19, F16, 9, (40, 40, 40), 0),
+    (19, F16, 9, (48, 48, 48), 1), (19, F16, 9, (64, 64, 32), 1), (19, F16, 9, (56, 56, 56), 0),
+    (19, F16, 9, (64, 64, 64), 1), (19, F16, 9, (192, 192, 192), 1), (19, BF16, 12, (32, 32, 32), 0),
+    (19, BF16, 12, (48, 48, 48), 0), (19, BF16, 12, (64, 64, 32), 1), (19, E3M12, 10, (32, 32, 32), 0),
+    (19, E3M12, 10, (64, 64, 64), 0), (19, E3M12, 10, (72, 72, 72), 0), (19, E3M12, 10, (80, 80, 80), 1),
+    (19, Q15, 10, (64, 64, 64), 0), (19, Q15, 10, (64, 64, 36), 1), (19, Q15, 10, (52, 52, 52), 0),
+    (19, F16, 9, (52, 52, 52), 1), (19, Q15, 10, (192, 96, 48), 1), (19, F16, 9, (128, 2, 1024), 0),
+    (19, F16, 9, (4, 4, 16384), 0), (19, F16, 9, (40, 40, 200), 0),
+    (9, F16, 16, (128, 128, 1), 0), (9, F16, 16, (256, 256, 1), 0), (9, F16, 16, (384, 384, 1), 1),
+    (9, F16, 16, (512, 512, 1), 1), (9, E3M12, 12, (256, 256, 1), 0), (9, E3M12, 12, (512, 512, 1), 0),
+    (9, E3M12, 12, (768, 768, 1), 1), (9, Q15, 16, (640, 640, 1), 0), (9, Q15, 16, (768, 768, 1), 1),
+    (9, F16, 0, (1024, 1024, 1), 1), (9, F16, 0, (128, 128, 1), 0),
+]
+
+
+def test_coupled_16bit_step(ask):
+    got = ask(["coupled %d %d %d %d %d %d" % (l, f, r, *b) for l, f, r, b, _ in COUPLED])
+    assert [g[0] for g in got] == [c[-1] for c in COUPLED]
