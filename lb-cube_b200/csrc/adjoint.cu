@@ -152,17 +152,18 @@ cudaError_t launch_adjoint_step(int collision, const Real* fn, const Real* lam_n
                                 cudaStream_t s) {
   // programmatic dependent launches (the kernel opens with pdl_enter)
   if constexpr (std::is_same_v<Real, float> && L::Q <= 19) {
-    if (pairs_eligible(g, 0, fn, lam_next, lam)) {
+    auto pairs = [&](auto ct) { return pairs_eligible<true>(g, kAdjointPairRule<L, decltype(ct)::value>, fn, lam_next, lam); };
+    auto run = [&](auto ct) {
       const PairGrid pg = make_pair_grid(g);
-      auto run = [&](auto ct) {
-        return launch_pdl(adjoint_step_pair_kernel<L, decltype(ct)::value>, pair_grid_dims(pg, g.nz),
-                          dim3(kThreads), 0, s, fn, lam_next, lam, pg, ap, dtau_slots);
-      };
-      if (collision == kBGK) return run(std::integral_constant<int, kBGK>{});
-      if (collision == kTRT) return run(std::integral_constant<int, kTRT>{});
-      if (collision == kMRT) return run(std::integral_constant<int, kMRT>{});
-      return cudaErrorInvalidValue;
-    }
+      return launch_pdl(adjoint_step_pair_kernel<L, decltype(ct)::value>, pair_grid_dims(pg, g.nz),
+                        dim3(kThreads), 0, s, fn, lam_next, lam, pg, ap, dtau_slots);
+    };
+    using B = std::integral_constant<int, kBGK>;
+    using T = std::integral_constant<int, kTRT>;
+    using M = std::integral_constant<int, kMRT>;
+    if (collision == kBGK && pairs(B{})) return run(B{});
+    if (collision == kTRT && pairs(T{})) return run(T{});
+    if (collision == kMRT && pairs(M{})) return run(M{});
   }
   const dim3 grid = grid_dims(g), block(block_dims(g));
   if (collision == kBGK)

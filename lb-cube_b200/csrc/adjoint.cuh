@@ -38,6 +38,19 @@ constexpr int kAdjointBlocks = sizeof(Real) == 4 ? 5 : 2;
 // resident blocks: 3.37, 3.25 and 3.52 ms (one cell per thread: 3.59).
 constexpr int kAdjointPairBlocks = 4;
 
+// From how many one-cell blocks per SM on the fluid adjoint step takes pairs. One
+// step in us, one cell -> two, at blocks per SM: D3Q19 BGK 24^3 (0.8) 2.6 -> 3.2, 44^3
+// (4.8) 5.0 -> 5.5, 48^3 (5.8) 6.4 -> 5.4, 64^3 (13.8) 10.6 -> 8.7, and within half of
+// either kernel's resident blocks (5 and 4) 40^3 (3.4) 4.9 -> 4.3. MRT, whose two
+// cells spill, 64^3 14.9 -> 15.7, 72^3 (19.9) 21.7 -> 23.0, 80^3 (27) 32.5 -> 31.0; past the
+// second wave of one cell but within the first of two, 52^3 (7.7) 10.0 -> 9.5. D2Q9:
+// 256^2 (3.5) BGK 2.5 -> 2.8, MRT 3.2 -> 3.4; 272^2 (3.9) TRT 3.9 -> 2.7, MRT 4.3 -> 3.3;
+// 384^2 (7.8) MRT 5.8 -> 4.6.
+template <class L, int CT>
+constexpr CellRule kAdjointPairRule = L::Q == 9      ? CellRule{3.7}
+                                      : CT == kMRT ? CellRule{22, 7.2, 4}
+                                                   : CellRule{5, 2.5, 2};
+
 struct AdjointParams {
   double omega, omega_minus;
   double domega_dtau, domega_minus_dtau;  // derivatives of the rates w.r.t. tau

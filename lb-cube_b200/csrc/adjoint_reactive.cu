@@ -347,6 +347,7 @@ __global__ void __launch_bounds__(kThreads, kAdjointBlocks<Real>)
 // (native 128^3 gradient 3.13 ms, 3.20 at 5, 3.28 at 6). Each warp adds to the slots of the first
 // of the one-cell blocks that its block covers.
 constexpr int kReactionPairBlocks = 4;
+constexpr CellRule kReactivePairRule{12};
 
 __device__ __forceinline__ long long pair_warp_slot(const PairGrid& g, int z) {
   return ((long long)z * g.tiles + (long long)kPairCells * blockIdx.x) * kWarpsPerBlock + (long long)(threadIdx.x >> 5);
@@ -558,7 +559,7 @@ cudaError_t launch_reactive_adjoint(int collision, int planes, const typename SP
                                     cudaStream_t s) {
   // programmatic dependent launches (the kernels open with pdl_enter)
   if constexpr (std::is_same_v<Real, float> && FL::Q <= 19) {
-    if (pairs_eligible(g, 12, fn, an, bn, u_next, lf_next, la_next, lb_next, lf, la, lb, ubar)) {
+    if (pairs_eligible<false>(g, kReactivePairRule, fn, an, bn, u_next, lf_next, la_next, lb_next, lf, la, lb, ubar)) {
       const PairGrid pg = make_pair_grid(g, g.z0);
       const dim3 grid = pair_grid_dims(pg, planes), block(kThreads);
       const cudaError_t err = launch_pdl(reaction_adjoint_pair_kernel<FL, SP>, grid, block, 0, s, an, bn, u_next,

@@ -139,7 +139,7 @@ constexpr int kCoupledPairBlocks = FL::Q == 19 ? 7 : 0;
 template <class FL, class Real>
 constexpr bool kAdrPairs = std::is_same_v<Real, float> && FL::Q <= 19;
 template <class FL>
-constexpr int kAdrPairFrom = FL::Q == 19 ? 12 : 16;
+constexpr CellRule kAdrPairRule{FL::Q == 19 ? 12.0 : 16.0};
 
 template <class FL>
 __global__ void __launch_bounds__(kThreads)
@@ -245,7 +245,7 @@ cudaError_t launch_coupled_step(const Grid& g, int planes, const Real* cur_f, Re
                                 Real omega_c, Real k, double* partials, Real* u_out, cudaStream_t s) {
   // programmatic dependent launches (the kernels open with pdl_enter)
   if constexpr (kAdrPairs<FL, Real>) {
-    if (pairs_eligible(g, kAdrPairFrom<FL>, cur_f, nxt_f, cur_a, nxt_a, cur_b, nxt_b, u_out)) {
+    if (pairs_eligible<STATS>(g, kAdrPairRule<FL>, cur_f, nxt_f, cur_a, nxt_a, cur_b, nxt_b, u_out)) {
       const PairGrid pg = make_pair_grid(g, g.z0);
       const dim3 grid = pair_grid_dims(pg, planes);
       using SL = typename ScalarOf<FL>::type;
@@ -469,7 +469,7 @@ cudaError_t launch_scalar(const Real* cur_s, Real* nxt_s, const Real* cur_f, siz
   const Span writes[1] = {{nxt_s, sb}};
   if (any_overlap(reads, writes)) return cudaErrorInvalidValue;
   if constexpr (kAdrPairs<FL, Real>) {
-    if (pairs_eligible(g, kAdrPairFrom<FL>, cur_s, nxt_s, cur_f)) {
+    if (pairs_eligible<false>(g, kAdrPairRule<FL>, cur_s, nxt_s, cur_f)) {
       const PairGrid pg = make_pair_grid(g);
       return launch_pdl(scalar_step_pair_kernel<FL>, pair_grid_dims(pg, g.nz), dim3(kThreads), 0, stream, cur_s,
                         nxt_s, cur_f, pg, omega_c, source);
@@ -496,7 +496,7 @@ cudaError_t launch_reaction(const Real* cur_a, Real* nxt_a, const Real* cur_b, R
   const Span writes[2] = {{nxt_a, sb}, {nxt_b, sb}};
   if (any_overlap(reads, writes)) return cudaErrorInvalidValue;
   if constexpr (kAdrPairs<FL, Real>) {
-    if (pairs_eligible(g, kAdrPairFrom<FL>, cur_a, nxt_a, cur_b, nxt_b, cur_f)) {
+    if (pairs_eligible<false>(g, kAdrPairRule<FL>, cur_a, nxt_a, cur_b, nxt_b, cur_f)) {
       const PairGrid pg = make_pair_grid(g);
       return launch_pdl(reaction_ab_pair_kernel<FL>, pair_grid_dims(pg, g.nz), dim3(kThreads), 0, stream, cur_a,
                         nxt_a, cur_b, nxt_b, cur_f, pg, omega_c, k);

@@ -40,12 +40,12 @@ inline dim3 pair_grid_dims(const PairGrid& p, int planes) {
 }
 
 // Rows of whole words in word-aligned buffers (an even plane keeps every
-// population plane aligned), and a box whose one-cell launch is more than
-// `per_sm` blocks on each of the 148 SMs: while that launch still fits the SMs at
-// once, its twice as many threads hide more latency than pairs save.
-template <class... P>
-inline bool pairs_eligible(const Grid& g, int per_sm, const P*... p) {
-  return g.nx % 2 == 0 && g.launched() > 148LL * per_sm && ((((uintptr_t)p % 8) == 0) && ...);
+// population plane aligned), and a box that the rule takes. REDUCES: the kernel
+// ends in a sum over the block.
+template <bool REDUCES, class... P>
+inline bool pairs_eligible(const Grid& g, const CellRule& rule, const P*... p) {
+  return g.nx % 2 == 0 && ((((uintptr_t)p % 8) == 0) && ...) &&
+         several_cells_pay(g.nx, g.ny, g.nz, kPairCells, REDUCES ? kThreads : 32, rule);
 }
 
 __device__ __forceinline__ bool pair_of(const PairGrid& g, int& x0, int& y, int& z) {

@@ -147,7 +147,7 @@ constexpr bool kUsePairs = sizeof(Real) == 4;
 // 72^3 18.0 -> 18.4, 88^3 (36) 36.6 -> 33.7; and its MRT: 60 x 62 x 64 (13.4) 11.9 ->
 // 12.4, 72^3 17.7 -> 18.0, 88 x 90 x 86 (35) 30.8 -> 29.4.
 template <class L, int CT>
-constexpr int kPairFrom = L::Q == 19 ? 12 : L::Q == 27 && (CT == kRLBM || CT == kMRT) ? 30 : 16;
+constexpr CellRule kPairRule{L::Q == 19 ? 12.0 : L::Q == 27 && (CT == kRLBM || CT == kMRT) ? 30.0 : 16.0};
 
 template <class L, int CT, bool DIAG, bool FIRST>
 __global__ void __launch_bounds__(kThreads, kPairBlocks<L, CT>)
@@ -180,7 +180,7 @@ inline cudaError_t launch_step(const Grid& g, int planes, const Real* cur, Real*
                                Real omega_minus, double* partials, long long* count, cudaStream_t s) {
   // programmatic dependent launches (the kernels open with pdl_enter)
   if constexpr (kUsePairs<L, Real, CT>) {
-    if (pairs_eligible(g, kPairFrom<L, CT>, cur, nxt)) {
+    if (pairs_eligible<DIAG>(g, kPairRule<L, CT>, cur, nxt)) {
       const PairGrid pg = make_pair_grid(g, g.z0);
       const dim3 grid = pair_grid_dims(pg, planes);
       if constexpr (DIAG) *count = (long long)grid.x * planes;

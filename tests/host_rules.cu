@@ -1,15 +1,25 @@
 // Test helper: answers questions about the host side of the kernels' launch rules,
 // one per line of standard input, from the engine's own headers.
 //   div n d            n / d through FastDiv
-//   coupled L FMT RESIDENT nx ny nz    1 if the 16-bit coupled step takes four cells per thread
-// (L: 9 or 19; FMT: 0 FP16, 1 BF16, 2 E3M12, 3 Q15; RESIDENT: blocks of its one-cell kernel per SM)
+//   adjoint L OP nx ny nz       1 if the FP32 adjoint step takes two cells per thread
+//   coupled L FMT RESIDENT nx ny nz    1 if the 16-bit coupled step takes four
+// (L: 9 or 19; OP: 0 BGK, 1 TRT, 2 MRT; FMT: 0 FP16, 1 BF16, 2 E3M12, 3 Q15; RESIDENT: blocks of its one-cell kernel per SM)
 #include <cstdio>
 #include <cstring>
 
+#include "../lb-cube_b200/csrc/adjoint.cuh"
+#include "../lb-cube_b200/csrc/pairs.cuh"
 #include "../lb-cube_b200/csrc/stream_codes.cuh"
 
 using namespace lbcube;
 
+template <class L>
+int adjoint_of(int op, const Grid& g) {
+  const float* p = (const float*)0x100;
+  return op == 0   ? pairs_eligible<true>(g, kAdjointPairRule<L, 0>, p)
+         : op == 1 ? pairs_eligible<true>(g, kAdjointPairRule<L, 1>, p)
+                   : pairs_eligible<true>(g, kAdjointPairRule<L, 2>, p);
+}
 template <class L>
 int coupled_of(int fmt, int resident, const Grid& g) {
   const CellRule r = fmt == kF16S    ? coupled_codes_rule<L, kF16S>(resident)
@@ -29,12 +39,14 @@ int main() {
     }
     int a[3];
     size_t n[3];
-    for (int& v : a)
-      if (scanf("%d", &v) != 1) return 2;
+    const int extra = strcmp(what, "adjoint") == 0 ? 2 : 3;
+    for (int i = 0; i < extra; ++i)
+      if (scanf("%d", &a[i]) != 1) return 2;
     if (scanf("%zu %zu %zu", &n[0], &n[1], &n[2]) != 3) return 2;
     Grid g{};
     if (validate_domain(false, 1, 1, 1, n[2] == 1 ? 2 : 3, n[0], n[1], n[2], g) != cudaSuccess) return 3;
-    printf("%d\n", a[0] == 9 ? coupled_of<D2Q9>(a[1], a[2], g) : coupled_of<D3Q19>(a[1], a[2], g));
+    if (extra == 2) printf("%d\n", a[0] == 9 ? adjoint_of<D2Q9>(a[1], g) : adjoint_of<D3Q19>(a[1], g));
+    else printf("%d\n", a[0] == 9 ? coupled_of<D2Q9>(a[1], a[2], g) : coupled_of<D3Q19>(a[1], a[2], g));
   }
   return 0;
 }

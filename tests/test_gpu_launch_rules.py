@@ -3,7 +3,15 @@ at boxes that reach them.
 
 * 16-bit coupled step, four cells per thread: the same state in buffers one code
   off the word alignment takes one cell per thread; the same codes bit for bit, the
-  same statistics to 1e-12 (FP64 sums of the same terms in another order)."""
+  same statistics to 1e-12 (FP64 sums of the same terms in another order).
+* FP32 adjoint step, two cells per thread: against the one-cell kernel on buffers one
+  element off the alignment. lambda to 1e-6. dJ/dtau slot by slot: a pair's block
+  adds the terms of 256 cells to the slot of the first of the two one-cell blocks
+  that it covers. A cell's term is a sum of products lambda_i times a relaxed difference
+  of f_i, formed in FP32 with at most 2e-6 of s = sum |lambda_i| |f_i| between two
+  orders of contraction (19 roundings of 2^-24 each on either side); over the cells of
+  a slot the differences add like independent ones, so the bar is six times 2e-6 of the
+  root of the sum of their s^2 (one missing cell, about 1e-2, is 50 times that)."""
 import numpy as np
 import pytest
 import torch
@@ -56,3 +64,30 @@ def test_coupled_words_match_single_cells(engine, dev, fl, fmt, op, dims, stats)
     if stats:
         assert bool(torch.isfinite(rows[0][1]).all())
         assert float(((rows[0][1] - rows[1][1]).abs() / rows[1][1].abs().clamp_min(1e-2)).max()) <= 1e-12
+
+
+@pytest.mark.parametrize("lat,op,dims", [("D3Q19", "BGK", (66, 62, 60)), ("D3Q19", "TRT", (50, 48, 52)),
+                                         ("D3Q19", "MRT", (82, 80, 76)), ("D2Q9", "TRT", (274, 273, 1)),
+                                         ("D2Q9", "MRT", (602, 301, 1)), ("D2Q9", "BGK", (514, 230, 1))])
+def test_adjoint_pairs_slot_by_slot(engine, dev, lat, op, dims):
+    nx, ny, nz = dims
+    f = torch.from_numpy(U.random_state(lat, *dims, np.float32, seed=64)).to(dev)
+    lam = torch.randn(f.shape, generator=torch.Generator(device=dev).manual_seed(65), device=dev)
+    count = engine.stats_partials_bytes(lat, *dims) // 40
+    got = []
+    for aligned in (True, False):
+        cur, nxt, out = (f, lam, torch.empty_like(f)) if aligned else (_off(f), _off(lam), _off(f))
+        tau = torch.zeros(count, dtype=torch.float64, device=dev)
+        engine.check(engine.adjoint_step_async(lat, "float", op, cur, nxt, out, *dims, 0.7, tau))
+        got.append((out.double(), tau))
+    torch.cuda.synchronize()
+    (a, pair), (b, one) = got
+    assert float((a - b).norm() / b.norm()) <= 1e-6
+    tiles = -(-nx * ny // 128)
+    pad = tiles % 2
+    one = torch.nn.functional.pad(one[:tiles * nz].view(nz, tiles), (0, pad)).view(nz, -1, 2)
+    pair = torch.nn.functional.pad(pair[:tiles * nz].view(nz, tiles), (0, pad)).view(nz, -1, 2)
+    assert float(pair[..., 1].abs().max()) == 0.0
+    s = (lam.double().abs() * f.double().abs()).sum(0).view(nz, nx * ny)
+    s2 = torch.nn.functional.pad(s * s, (0, 256 * one.shape[1] - nx * ny)).view(nz, -1, 256).sum(-1)
+    assert bool(((pair[..., 0] - one.sum(-1)).abs() <= 6 * 2e-6 * s2.sqrt()).all())

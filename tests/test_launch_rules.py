@@ -14,6 +14,7 @@ import pytest
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 NVCC = os.environ.get("NVCC", shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc")
+BGK, TRT, MRT, RLBM = range(4)
 F16, BF16, E3M12, Q15 = range(4)
 
 
@@ -68,3 +69,17 @@ COUPLED = [
 def test_coupled_16bit_step(ask):
     got = ask(["coupled %d %d %d %d %d %d" % (l, f, r, *b) for l, f, r, b, _ in COUPLED])
     assert [g[0] for g in got] == [c[-1] for c in COUPLED]
+
+
+ADJOINT = [
+    (19, BGK, (16, 16, 16), 0), (19, TRT, (24, 24, 24), 0), (19, BGK, (32, 32, 32), 0), (19, BGK, (40, 40, 40), 1),
+    (19, TRT, (44, 44, 44), 0), (19, TRT, (48, 48, 48), 1), (19, BGK, (128, 128, 128), 1), (19, MRT, (32, 32, 32), 0),
+    (19, MRT, (64, 64, 64), 0), (19, MRT, (52, 52, 52), 1), (19, MRT, (80, 80, 80), 1), (19, BGK, (8, 8, 4096), 0),
+    (19, MRT, (4, 4, 16384), 0), (19, BGK, (65, 64, 64), 0),
+    (9, BGK, (128, 128, 1), 0), (9, MRT, (256, 256, 1), 0), (9, TRT, (272, 272, 1), 1), (9, MRT, (512, 512, 1), 1),
+]
+
+
+def test_adjoint_step(ask):
+    got = ask(["adjoint %d %d %d %d %d" % (l, op, *b) for l, op, b, _ in ADJOINT])
+    assert [g[0] for g in got] == [c[-1] for c in ADJOINT]
