@@ -138,19 +138,26 @@ __global__ void __launch_bounds__(kThreads)
 // 83.6 us against 92 at 3 and 86 at 5, which spills).
 template <class L, int CT>
 constexpr int kPairBlocks = L::Q == 27 && CT == kMRT ? 4 : L::Q == 19 && CT != kRLBM ? 7 : 0;
-template <class L, class Real, int CT>
-constexpr bool kUsePairs = sizeof(Real) == 4;
-// From how many one-cell blocks per SM on (pairs_eligible): what the SMs hold
-// at once. D3Q19 12: MRT 56^3 (9.3 blocks per SM) 6.6 -> 7.1 us, 64^3 (13.8) 7.7 ->
-// 6.8. D2Q9 16: MRT 512^2 (13.8) 4.2 -> 5.2, 600^2 (19) 5.1 -> 5.0, 724^2 6.5 -> 5.8.
-// D3Q27 likewise: BGK 64^3 (13.8) level, 72^3 (19.7) 11.5 -> 10.4; its RLBM later:
-// 72^3 18.0 -> 18.4, 88^3 (36) 36.6 -> 33.7; and its MRT: 60 x 62 x 64 (13.4) 11.9 ->
-// 12.4, 72^3 17.7 -> 18.0, 88 x 90 x 86 (35) 30.8 -> 29.4.
+// From how many one-cell blocks per SM on: what the SMs hold at once. D3Q19 12:
+// MRT 56^3 (9.5 blocks per SM) 6.1 -> 6.5 us, 64^3 (13.8) 7.3 -> 6.6. D2Q9 16: MRT
+// 512^2 (13.8) 4.2 -> 5.2, 600^2 (19) 5.1 -> 5.0, 724^2 6.5 -> 5.8. D3Q27 likewise:
+// BGK 64^3 (13.8) level, 72^3 (19.9) 11.5 -> 10.4; its RLBM later: 72^3 18.0 -> 18.4,
+// 88^3 (36) 36.6 -> 33.7; and its MRT: 60 x 62 x 64 (13.4) 11.9 -> 12.4, 72^3 17.7 ->
+// 18.0, 88 x 90 x 86 (35) 30.8 -> 29.4. Between, D3Q19 BGK, TRT and MRT: from 6 (half of
+// the 12 resident one-cell blocks) while the pairs' blocks stay within half of their
+// 7: 64 x 64 x 32 (6.9) BGK 4.8 -> 3.8, TRT 5.2 -> 4.0, MRT 5.3 -> 4.5; BGK and TRT up to
+// half of 8, on a kernel of that budget (64 registers, 6 % slower where both fit):
+// 64 x 64 x 36 BGK 4.95 -> 4.1, 52^3 TRT 5.3 -> 4.2.
+constexpr int kWindowBlocks = 8;
 template <class L, int CT>
-constexpr CellRule kPairRule{L::Q == 19 ? 12.0 : L::Q == 27 && (CT == kRLBM || CT == kMRT) ? 30.0 : 16.0};
+constexpr CellRule kPairRule = L::Q != 19 ? CellRule{L::Q == 27 && (CT == kRLBM || CT == kMRT) ? 30.0 : 16.0}
+                               : CT == kRLBM ? CellRule{12}
+                                             : CellRule{12, 6, CT == kMRT ? 3.5 : kWindowBlocks / 2.0};
+template <class L, class Real, bool DIAG>
+constexpr bool kUsePairs = sizeof(Real) == 4;
 
-template <class L, int CT, bool DIAG, bool FIRST>
-__global__ void __launch_bounds__(kThreads, kPairBlocks<L, CT>)
+template <class L, int CT, bool DIAG, bool FIRST, int BLOCKS>
+__global__ void __launch_bounds__(kThreads, BLOCKS)
     fluid_step_pair_kernel(const float* __restrict__ cur, float* __restrict__ nxt, PairGrid g, float omega,
                            float omega_minus, double* __restrict__ partials) {
   pdl_enter();
@@ -179,13 +186,21 @@ template <class L, class Real, int CT, bool DIAG, bool FIRST>
 inline cudaError_t launch_step(const Grid& g, int planes, const Real* cur, Real* nxt, Real omega,
                                Real omega_minus, double* partials, long long* count, cudaStream_t s) {
   // programmatic dependent launches (the kernels open with pdl_enter)
-  if constexpr (kUsePairs<L, Real, CT>) {
+  if constexpr (kUsePairs<L, Real, DIAG>) {
     if (pairs_eligible<DIAG>(g, kPairRule<L, CT>, cur, nxt)) {
       const PairGrid pg = make_pair_grid(g, g.z0);
       const dim3 grid = pair_grid_dims(pg, planes);
       if constexpr (DIAG) *count = (long long)grid.x * planes;
-      return launch_pdl(fluid_step_pair_kernel<L, CT, DIAG, FIRST>, grid, dim3(kThreads), 0, s, cur, nxt, pg,
-                        omega, omega_minus, partials);
+      auto run = [&](auto blocks) {
+        return launch_pdl(fluid_step_pair_kernel<L, CT, DIAG, FIRST, decltype(blocks)::value>, grid, dim3(kThreads), 0,
+                          s, cur, nxt, pg, omega, omega_minus, partials);
+      };
+      if constexpr (kPairRule<L, CT>.hi == kWindowBlocks / 2.0 && !FIRST) {
+        const bool window = g.launched() <= (long long)kPairRule<L, CT>.from * kSMs;
+        if (window && 2LL * grid.x * planes > (long long)kPairBlocks<L, CT> * kSMs)
+          return run(std::integral_constant<int, kWindowBlocks>{});
+      }
+      return run(std::integral_constant<int, kPairBlocks<L, CT>>{});
     }
   }
   const dim3 grid((unsigned)g.tiles, (unsigned)planes), block(block_dims(g));

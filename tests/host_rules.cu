@@ -1,18 +1,29 @@
 // Test helper: answers questions about the host side of the kernels' launch rules,
 // one per line of standard input, from the engine's own headers.
 //   div n d            n / d through FastDiv
-//   adjoint L OP nx ny nz       1 if the FP32 adjoint step takes two cells per thread
+//   fluid L OP DIAG nx ny nz    1 if the FP32 fluid step takes two cells per thread
+//   adjoint L OP nx ny nz       the same for the FP32 adjoint step
 //   coupled L FMT RESIDENT nx ny nz    1 if the 16-bit coupled step takes four
-// (L: 9 or 19; OP: 0 BGK, 1 TRT, 2 MRT; FMT: 0 FP16, 1 BF16, 2 E3M12, 3 Q15; RESIDENT: blocks of its one-cell kernel per SM)
+// (L: 9, 19 or 27; OP: 0 BGK, 1 TRT, 2 MRT, 3 RLBM; FMT: 0 FP16, 1 BF16, 2 E3M12, 3 Q15; RESIDENT: blocks of its one-cell kernel per SM)
 #include <cstdio>
 #include <cstring>
 
 #include "../lb-cube_b200/csrc/adjoint.cuh"
-#include "../lb-cube_b200/csrc/pairs.cuh"
+#include "../lb-cube_b200/csrc/step_cell.cuh"
 #include "../lb-cube_b200/csrc/stream_codes.cuh"
 
 using namespace lbcube;
 
+template <class L, int OP, bool DIAG>
+int fluid(const Grid& g) {
+  return kUsePairs<L, float, DIAG> && pairs_eligible<DIAG>(g, kPairRule<L, OP>, (float*)0x100);
+}
+template <class L>
+int fluid_of(int op, int diag, const Grid& g) {
+  const int v[4][2] = {{fluid<L, 0, false>(g), fluid<L, 0, true>(g)}, {fluid<L, 1, false>(g), fluid<L, 1, true>(g)},
+                       {fluid<L, 2, false>(g), fluid<L, 2, true>(g)}, {fluid<L, 3, false>(g), fluid<L, 3, true>(g)}};
+  return v[op][diag];
+}
 template <class L>
 int adjoint_of(int op, const Grid& g) {
   const float* p = (const float*)0x100;
@@ -46,6 +57,10 @@ int main() {
     Grid g{};
     if (validate_domain(false, 1, 1, 1, n[2] == 1 ? 2 : 3, n[0], n[1], n[2], g) != cudaSuccess) return 3;
     if (extra == 2) printf("%d\n", a[0] == 9 ? adjoint_of<D2Q9>(a[1], g) : adjoint_of<D3Q19>(a[1], g));
+    else if (strcmp(what, "fluid") == 0)
+      printf("%d\n", a[0] == 9    ? fluid_of<D2Q9>(a[1], a[2], g)
+                     : a[0] == 19 ? fluid_of<D3Q19>(a[1], a[2], g)
+                                  : fluid_of<D3Q27>(a[1], a[2], g));
     else printf("%d\n", a[0] == 9 ? coupled_of<D2Q9>(a[1], a[2], g) : coupled_of<D3Q19>(a[1], a[2], g));
   }
   return 0;

@@ -11,7 +11,9 @@ at boxes that reach them.
   of f_i, formed in FP32 with at most 2e-6 of s = sum |lambda_i| |f_i| between two
   orders of contraction (19 roundings of 2^-24 each on either side); over the cells of
   a slot the differences add like independent ones, so the bar is six times 2e-6 of the
-  root of the sum of their s^2 (one missing cell, about 1e-2, is 50 times that)."""
+  root of the sum of their s^2 (one missing cell, about 1e-2, is 50 times that).
+* FP32 D3Q19 step and diagnostics in the range where the pairs run in 7 or 8 blocks
+  per SM: against the CPU oracle, bit for bit (diagnostics 1e-12)."""
 import numpy as np
 import pytest
 import torch
@@ -91,3 +93,25 @@ def test_adjoint_pairs_slot_by_slot(engine, dev, lat, op, dims):
     s = (lam.double().abs() * f.double().abs()).sum(0).view(nz, nx * ny)
     s2 = torch.nn.functional.pad(s * s, (0, 256 * one.shape[1] - nx * ny)).view(nz, -1, 256).sum(-1)
     assert bool(((pair[..., 0] - one.sum(-1)).abs() <= 6 * 2e-6 * s2.sqrt()).all())
+
+
+STEPS = [("D3Q19", "float", "BGK", (64, 64, 32)), ("D3Q19", "float", "TRT", (52, 50, 54)),
+         ("D3Q19", "float", "MRT", (48, 48, 56))]
+
+
+@pytest.mark.parametrize("lat,real,op,dims", STEPS)
+def test_steps(engine, dev, lat, real, op, dims):
+    f0 = U.random_state(lat, *dims, np.float32 if real == "float" else np.float64, seed=66)
+    cur = torch.from_numpy(f0).to(dev)
+    nxt, again = torch.empty_like(cur), torch.empty_like(cur)
+    nbytes = engine.diagnostics_partials_bytes(lat, *dims)
+    part = torch.full((nbytes // 8,), float("nan"), dtype=torch.float64, device=dev)
+    out = torch.empty(5, dtype=torch.float64, device=dev)
+    engine.check(engine.step_async(lat, real, op, cur, nxt, *dims, 1 / 0.6))
+    engine.check(engine.step_diagnostics_async(lat, real, op, cur, again, *dims, 1 / 0.6, part, nbytes, out))
+    torch.cuda.synchronize()
+    want = O.step(f0, lat, op, *dims, 1 / 0.6, steps=1)
+    assert U.same_bits(nxt.cpu().numpy(), want)
+    assert U.same_bits(again.cpu().numpy(), want)
+    for g, w in zip(out.cpu().numpy()[:3], O.fluid_diagnostics64(want, lat, *dims)[:3]):
+        assert abs(g - w) <= 1e-12 * max(abs(w), 1e-6)

@@ -83,3 +83,19 @@ ADJOINT = [
 def test_adjoint_step(ask):
     got = ask(["adjoint %d %d %d %d %d" % (l, op, *b) for l, op, b, _ in ADJOINT])
     assert [g[0] for g in got] == [c[-1] for c in ADJOINT]
+
+
+FLUID = [
+    # lattice, operator, with diagnostics, box, two cells per thread
+    (19, BGK, 0, (64, 64, 32), 1), (19, TRT, 0, (64, 64, 32), 1), (19, TRT, 1, (64, 64, 32), 1),
+    (19, BGK, 0, (48, 48, 56), 1), (19, BGK, 0, (52, 52, 52), 1), (19, MRT, 0, (52, 52, 52), 0), (19, BGK, 0, (56, 56, 56), 0),
+    (19, BGK, 0, (64, 64, 64), 1), (19, BGK, 0, (32, 32, 32), 0), (19, RLBM, 0, (64, 64, 32), 0),
+    (19, RLBM, 0, (4, 4, 16384), 0), (27, RLBM, 0, (4, 4, 16384), 0), (27, RLBM, 0, (96, 96, 96), 1),
+    (27, BGK, 0, (96, 96, 96), 1),
+    (9, BGK, 0, (512, 512, 1), 0), (9, BGK, 1, (1024, 1024, 1), 1),
+]
+
+
+def test_fluid_step(ask):
+    got = ask(["fluid %d %d %d %d %d %d" % (l, op, d, *b) for l, op, d, b, _ in FLUID])
+    assert [g[0] for g in got] == [c[-1] for c in FLUID]
