@@ -153,8 +153,11 @@ template <class L, int CT>
 constexpr CellRule kPairRule = L::Q != 19 ? CellRule{L::Q == 27 && (CT == kRLBM || CT == kMRT) ? 30.0 : 16.0}
                                : CT == kRLBM ? CellRule{12}
                                              : CellRule{12, 6, CT == kMRT ? 3.5 : kWindowBlocks / 2.0};
+// The diagnostics form of the D3Q27 step keeps one cell per thread: its FP64 sums
+// cost a pair more registers than the saved loads are worth (96^3: TRT 41.7 us
+// against 43.2, MRT 54.6 against 56.9, RLBM 56.2 against 57.9).
 template <class L, class Real, bool DIAG>
-constexpr bool kUsePairs = sizeof(Real) == 4;
+constexpr bool kUsePairs = sizeof(Real) == 4 && !(DIAG && L::Q == 27);
 
 template <class L, int CT, bool DIAG, bool FIRST, int BLOCKS>
 __global__ void __launch_bounds__(kThreads, BLOCKS)

@@ -13,7 +13,8 @@ at boxes that reach them.
   a slot the differences add like independent ones, so the bar is six times 2e-6 of the
   root of the sum of their s^2 (one missing cell, about 1e-2, is 50 times that).
 * FP32 D3Q19 step and diagnostics in the range where the pairs run in 7 or 8 blocks
-  per SM: against the CPU oracle, bit for bit (diagnostics 1e-12)."""
+  per SM, and of D3Q27, whose diagnostics keep one cell per thread: against the CPU
+  oracle, bit for bit (diagnostics 1e-12)."""
 import numpy as np
 import pytest
 import torch
@@ -96,7 +97,7 @@ def test_adjoint_pairs_slot_by_slot(engine, dev, lat, op, dims):
 
 
 STEPS = [("D3Q19", "float", "BGK", (64, 64, 32)), ("D3Q19", "float", "TRT", (52, 50, 54)),
-         ("D3Q19", "float", "MRT", (48, 48, 56))]
+         ("D3Q19", "float", "MRT", (48, 48, 56)), ("D3Q27", "float", "TRT", (74, 70, 72))]
 
 
 @pytest.mark.parametrize("lat,real,op,dims", STEPS)

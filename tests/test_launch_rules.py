@@ -91,7 +91,7 @@ FLUID = [
     (19, BGK, 0, (48, 48, 56), 1), (19, BGK, 0, (52, 52, 52), 1), (19, MRT, 0, (52, 52, 52), 0), (19, BGK, 0, (56, 56, 56), 0),
     (19, BGK, 0, (64, 64, 64), 1), (19, BGK, 0, (32, 32, 32), 0), (19, RLBM, 0, (64, 64, 32), 0),
     (19, RLBM, 0, (4, 4, 16384), 0), (27, RLBM, 0, (4, 4, 16384), 0), (27, RLBM, 0, (96, 96, 96), 1),
-    (27, BGK, 0, (96, 96, 96), 1),
+    (27, BGK, 0, (96, 96, 96), 1), (27, TRT, 1, (96, 96, 96), 0), (27, RLBM, 1, (128, 128, 128), 0),
     (9, BGK, 0, (512, 512, 1), 0), (9, BGK, 1, (1024, 1024, 1), 1),
 ]
 
