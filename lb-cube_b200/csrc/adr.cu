@@ -111,8 +111,18 @@ __device__ __forceinline__ void fluid_reaction_body(const Real* __restrict__ cur
                                                  kStatSums);
 }
 
-template <class FL, class Real, int CT, bool STATS, bool UOUT = false>
-__global__ void __launch_bounds__(kThreads)
+// Resident blocks that the statistics forms' register allocation must allow (0:
+// the compiler's choice), the plain step's: D2Q9 FP32 40 registers instead of 44
+// (TRT 1023 x 1024, odd rows: 32.9 -> 31.2 us), D3Q27 FP64 TRT 128 instead of 134, four
+// blocks instead of three (96^3 108.6 -> 95.1 us, 32^3 6.8 -> 5.5), except between two and
+// three blocks per SM, which three hold at once (36^3 6.7, 7.7 at four).
+// The D2Q9 one costs boxes that fit the SMs at once (512^2 8.8 -> 9.2): from
+// kAdrPairRule's line on only.
+template <class FL, class Real, int CT, bool STATS>
+constexpr int kStatsBlocks = STATS && FL::Q == 27 && sizeof(Real) == 8 && CT == kTRT ? 4 : 0;
+
+template <class FL, class Real, int CT, bool STATS, bool UOUT = false, int BLOCKS = kStatsBlocks<FL, Real, CT, STATS>>
+__global__ void __launch_bounds__(kThreads, BLOCKS)
     fluid_reaction_kernel(const Real* __restrict__ cur_f, Real* __restrict__ nxt_f,
                           const Real* __restrict__ cur_a, Real* __restrict__ nxt_a,
                           const Real* __restrict__ cur_b, Real* __restrict__ nxt_b, Grid g,
@@ -259,9 +269,18 @@ cudaError_t launch_coupled_step(const Grid& g, int planes, const Real* cur_f, Re
                         nxt_f, cur_a, nxt_a, cur_b, nxt_b, pg, omega, omega_minus, omega_c, k, partials, u_out);
     }
   }
-  return launch_pdl(fluid_reaction_kernel<FL, Real, CT, STATS, UOUT>, dim3((unsigned)g.tiles, (unsigned)planes),
-                    dim3(block_dims(g)), 0, s, cur_f, nxt_f, cur_a, nxt_a, cur_b, nxt_b, g, omega, omega_minus,
-                    omega_c, k, partials, u_out);
+  auto run = [&](auto kernel) {
+    return launch_pdl(kernel, dim3((unsigned)g.tiles, (unsigned)planes), dim3(block_dims(g)), 0, s, cur_f, nxt_f,
+                      cur_a, nxt_a, cur_b, nxt_b, g, omega, omega_minus, omega_c, k, partials, u_out);
+  };
+  if constexpr (STATS && FL::Q == 9 && sizeof(Real) == 4) {
+    if ((double)g.launched() > kAdrPairRule<FL>.from * kSMs) return run(fluid_reaction_kernel<FL, Real, CT, STATS, UOUT, 12>);
+  }
+  if constexpr (kStatsBlocks<FL, Real, CT, STATS> == 4) {
+    if (g.launched() > 2LL * kSMs && g.launched() <= 3LL * kSMs)
+      return run(fluid_reaction_kernel<FL, Real, CT, STATS, UOUT, 0>);
+  }
+  return run(fluid_reaction_kernel<FL, Real, CT, STATS, UOUT>);
 }
 
 // ---- z-slab form of the coupled step ----------------------------------------

@@ -14,7 +14,9 @@ at boxes that reach them.
   root of the sum of their s^2 (one missing cell, about 1e-2, is 50 times that).
 * FP32 D3Q19 step and diagnostics in the range where the pairs run in 7 or 8 blocks
   per SM, and of D3Q27, whose diagnostics keep one cell per thread: against the CPU
-  oracle, bit for bit (diagnostics 1e-12)."""
+  oracle, bit for bit (diagnostics 1e-12).
+* Coupled step with statistics on the kernels with register budgets: against the
+  step without, bit for bit, and the statistics of the fields it wrote, 1e-12."""
 import numpy as np
 import pytest
 import torch
@@ -116,3 +118,31 @@ def test_steps(engine, dev, lat, real, op, dims):
     assert U.same_bits(again.cpu().numpy(), want)
     for g, w in zip(out.cpu().numpy()[:3], O.fluid_diagnostics64(want, lat, *dims)[:3]):
         assert abs(g - w) <= 1e-12 * max(abs(w), 1e-6)
+
+
+@pytest.mark.parametrize("fl,real,op,dims", [("D3Q27", "double", "TRT", (33, 5, 7)), ("D3Q27", "double", "TRT", (36, 35, 33)),
+                                             ("D2Q9", "float", "TRT", (801, 799, 1))])
+def test_statistics(engine, dev, fl, real, op, dims):
+    """The fused statistics against those of the fields it wrote, in scratch of exactly
+    the public size, and the field against the step without statistics."""
+    dt, sl = np.float32 if real == "float" else np.float64, O.SCALAR_OF[fl]
+    state = [torch.from_numpy(x).to(dev) for x in (U.random_state(fl, *dims, dt, seed=67), U.random_scalar(sl, *dims, dt, seed=68),
+                                                   U.random_scalar(sl, *dims, dt, seed=69))]
+    nbytes = engine.stats_partials_bytes(fl, *dims)
+    runs = []
+    for stats in (True, False):
+        nxt = [torch.empty_like(t) for t in state]
+        part = torch.full((nbytes // 8 + 1,), float("nan"), dtype=torch.float64, device=dev)
+        part[-1] = 7.0
+        engine.check(engine.fluid_reaction_ab_async(fl, real, op, state[0], nxt[0], state[1], nxt[1], state[2], nxt[2], *dims,
+                                                    1 / 0.6, 1 / 0.8, 0.3, part if stats else None, nbytes if stats else 0))
+        runs.append((nxt, part))
+    out, ref = (torch.zeros(8, dtype=torch.float64, device=dev) for _ in range(2))
+    engine.check(engine.reactive_stats_finalize_async(fl, real, *dims, 0.3, runs[0][1], nbytes, out))
+    scratch = torch.empty(nbytes // 8, dtype=torch.float64, device=dev)
+    engine.check(engine.reactive_stats_async(sl, real, runs[0][0][1], runs[0][0][2], *dims, 0.3, scratch, nbytes, ref))
+    torch.cuda.synchronize()
+    for a, b in zip(runs[0][0], runs[1][0]):
+        assert U.same_bits(a.cpu().numpy(), b.cpu().numpy())
+    assert float(runs[0][1][-1]) == 7.0
+    assert float(((out - ref).abs() / ref.abs().clamp_min(1e-2)).max()) <= 1e-12
