@@ -165,16 +165,17 @@ cudaError_t launch_adjoint_step(int collision, const Real* fn, const Real* lam_n
     if (collision == kTRT && pairs(T{})) return run(T{});
     if (collision == kMRT && pairs(M{})) return run(M{});
   }
-  const dim3 grid = grid_dims(g), block(block_dims(g));
+  const Grid gl = latency_grid<L, Real>(g, kAdjointSpread);
+  const dim3 grid = grid_dims(gl), block(block_dims(gl));
   if (collision == kBGK)
-    return launch_pdl(adjoint_step_kernel<L, Real, kBGK>, grid, block, 0, s, fn, lam_next, lam, g, ap,
+    return launch_pdl(adjoint_step_kernel<L, Real, kBGK>, grid, block, 0, s, fn, lam_next, lam, gl, ap,
                       dtau_slots);
   if (collision == kTRT)
-    return launch_pdl(adjoint_step_kernel<L, Real, kTRT>, grid, block, 0, s, fn, lam_next, lam, g, ap,
+    return launch_pdl(adjoint_step_kernel<L, Real, kTRT>, grid, block, 0, s, fn, lam_next, lam, gl, ap,
                       dtau_slots);
   if constexpr (L::Q != 27) {
     if (collision != kMRT) return cudaErrorInvalidValue;
-    return launch_pdl(adjoint_step_kernel<L, Real, kMRT>, grid, block, 0, s, fn, lam_next, lam, g, ap,
+    return launch_pdl(adjoint_step_kernel<L, Real, kMRT>, grid, block, 0, s, fn, lam_next, lam, gl, ap,
                       dtau_slots);
   } else {
     return cudaErrorInvalidValue;
@@ -194,7 +195,7 @@ struct GradientLayout {
   long long ckpts;   // checkpoints stored (including the initial state)
   size_t off_ckpt, off_seg, off_lam, off_slots, total;
   long long slots;   // FP64 slots (room for every block)
-  long long used;    // slots that the launches write
+  long long used;    // slots that a launch in blocks of kThreads writes
 };
 
 inline GradientLayout gradient_layout(int Q, size_t elem, const Grid& g, int steps, int interval) {
@@ -276,7 +277,7 @@ cudaError_t ke_gradient(int collision, const Real* rho0, const Real* u0, const G
   err = launch_pdl(velocity_gradient_kernel<L, Real>, grid_dims(g), dim3(block_dims(g)), 0, s, rho0, u0,
                    (const Real*)lam[0], grad_u0, g);
   if (err != cudaSuccess) return err;
-  return launch_slot_sums(2, {{{ke_slots, lay.used, 1, 1.0, out}, {dtau_slots, lay.used, 1, 1.0, out + 1}}}, s);
+  return launch_slot_sums(2, {{{ke_slots, lay.used, 1, 1.0, out}, {dtau_slots, latency_grid<L, Real>(g, kAdjointSpread).launched(), 1, 1.0, out + 1}}}, s);
 }
 
 template <class Real>

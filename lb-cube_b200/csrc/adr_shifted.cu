@@ -293,8 +293,9 @@ cudaError_t launch_shifted_coupled(const unsigned short* cf, unsigned short* nf,
                                    double* partials, const Grid& g, float omega, float omega_c,
                                    float k, float rho0, float c0, cudaStream_t s) {
   const float om = CT == kTRT ? trt_omega_minus<float>(omega) : 0.0f;
-#define LBCUBE_SC(ST, UO)                                                                            \
-  return launch_coupled_planes<FL, FMT, CT, ST, UO>(cf, nf, ca, na, cb, nb, u_out, partials, g, 0, g.nz, \
+  const Grid gs = partials != nullptr ? stats_grid(g) : g;
+#define LBCUBE_SC(ST, UO)                                                                             \
+  return launch_coupled_planes<FL, FMT, CT, ST, UO>(cf, nf, ca, na, cb, nb, u_out, partials, gs, 0, g.nz, \
                                                     omega, om, omega_c, k, rho0, c0, s)
   if (partials != nullptr && u_out != nullptr) LBCUBE_SC(true, true);
   if (partials != nullptr) LBCUBE_SC(true, false);

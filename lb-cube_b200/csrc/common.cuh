@@ -212,6 +212,41 @@ inline cudaError_t validate_domain(bool any_null, unsigned bx, unsigned by, unsi
   return cudaSuccess;
 }
 
+// A grid of fewer than `below` blocks per SM with smaller blocks, whole warps, until it
+// has `upto` per SM, as far as the partials contract allows (launched() <= blocks()).
+// A small box is bound by latency: more and smaller blocks reach more SMs, and a
+// block's sums cross fewer warps; launches bound by neither lose to it (FP32 D3Q19
+// BGK step 32^3 2.1 -> 2.5 us).
+inline Grid spread(Grid g, double below, int upto) {
+  const long long cells = (long long)g.nx * g.ny;
+  auto launch_blocks = [&](int bx) { return (cells + bx - 1) / bx * g.nz; };
+  if ((double)g.launched() >= below * kSMs) return g;
+  while (g.bx > 32 && launch_blocks(g.bx) < (long long)upto * kSMs) {
+    const int smaller = (g.bx / 2 + 31) / 32 * 32;
+    if (launch_blocks(smaller) > g.row_blocks) break;
+    g.bx = smaller;
+  }
+  g.tiles = (int)((cells + g.bx - 1) / g.bx);
+  return g;
+}
+
+// The blocks of a statistics launch, whose partials the second pass counts from
+// the extents alone. Coupled step with statistics, blocks of 128 -> these, us: D3Q19
+// FP64 BGK 16^3 3.85 -> 3.25, 32^3 (1.7 blocks per SM) 4.70 -> 4.0, 40^3 (3.4) 7.0 -> 7.3
+// and so left alone; FP32 TRT 16^3 3.4 -> 3.0.
+inline Grid stats_grid(const Grid& g) { return spread(g, 2, 4); }
+
+// The blocks of a 3-D FP64 launch over a whole box without partials, planes of less
+// than a block apart (8^3 1.80 -> 1.88 us). Step, blocks of 128 -> these, us: D3Q27 BGK
+// 16^3 2.39 -> 2.14, 28^3 (1.3 blocks per SM) 3.16 -> 2.65, D3Q19 RLBM 28^3 3.5 -> 3.1; from
+// 32^3 (1.7) on level or slower, the adjoint already at 28^3 (D3Q27 BGK 4.4 -> 4.75,
+// 16^3 3.15 -> 2.8).
+constexpr double kStepSpread = 1.7, kAdjointSpread = 1;
+template <class L, class Real>
+inline Grid latency_grid(const Grid& g, double below) {
+  return sizeof(Real) == 8 && L::Q >= 19 && g.bx == kThreads ? spread(g, below, 3) : g;
+}
+
 // Whether the loads of a step mark their lines to be evicted first. Each
 // population is read once per step, so when the buffers read and written (bytes
 // in all) only just exceed the L2 (126 MB), giving up the lines already read

@@ -168,7 +168,7 @@ cudaError_t launch_finalize(const Grid& g, double k, const double* partials, dou
                             cudaStream_t s) {
   // programmatic dependent launches (the statistics kernels open with pdl_enter)
   return launch_pdl(stats_finalize_kernel, dim3(kFinalBlocks), dim3(kFinalThreads), 0, s, partials,
-                    g.launched(), (long long)g.plane, k, out);
+                    stats_grid(g).launched(), (long long)g.plane, k, out);
 }
 
 template <class SL, class Real>
@@ -187,7 +187,8 @@ cudaError_t launch_stats(const void* va, const void* vb, size_t nx, size_t ny, s
   const Span reads[2] = {{a, sb}, {b, sb}};
   const Span writes[2] = {{partials, need}, {out, 8 * sizeof(double)}};
   if (any_overlap(reads, writes)) return cudaErrorInvalidValue;
-  err = launch_pdl(stats_partials_kernel<SL, Real>, grid_dims(g), dim3(block_dims(g)), 0, s, a, b, g,
+  const Grid gs = stats_grid(g);
+  err = launch_pdl(stats_partials_kernel<SL, Real>, grid_dims(gs), dim3(block_dims(gs)), 0, s, a, b, gs,
                    partials);
   if (err != cudaSuccess) return err;
   // k_react has the population precision, as in compute_reactive_stats<SL, Real>.
@@ -267,7 +268,7 @@ extern "C" int lbm_reactive_stats_append_async(int fluid_lattice, int precision,
   if (any_overlap(reads, writes)) return (int)cudaErrorInvalidValue;
   const double k = precision == LBM_FLOAT ? (double)(float)k_react : k_react;
   return (int)launch_pdl(stats_append_kernel, dim3(kFinalBlocks), dim3(kFinalThreads), 0, as_stream(stream),
-                         (const double*)partials, g.launched(), (long long)g.plane, k, table,
+                         (const double*)partials, stats_grid(g).launched(), (long long)g.plane, k, table,
                          (unsigned long long)table_rows, row_counter);
 }
 
@@ -286,7 +287,7 @@ extern "C" int lbm_reactive_stats_sums_async(int fluid_lattice, size_t x_extent,
   if (err != cudaSuccess) return (int)err;
   if (partials_bytes < (size_t)g.blocks() * kStatSums * sizeof(double)) return (int)cudaErrorInvalidValue;
   return (int)launch_pdl(stats_sums_kernel, dim3(kFinalBlocks), dim3(kFinalThreads), 0, as_stream(stream),
-                         partials, g.launched(), sums);
+                         partials, stats_grid(g).launched(), sums);
 }
 
 extern "C" int lbm_reactive_stats_from_sums_async(int precision, const double* sums, double cells,

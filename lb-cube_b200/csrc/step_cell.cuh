@@ -206,14 +206,15 @@ inline cudaError_t launch_step(const Grid& g, int planes, const Real* cur, Real*
       return run(std::integral_constant<int, kPairBlocks<L, CT>>{});
     }
   }
-  const dim3 grid((unsigned)g.tiles, (unsigned)planes), block(block_dims(g));
+  const Grid gl = DIAG || planes != g.nz ? g : latency_grid<L, Real>(g, kStepSpread);
+  const dim3 grid((unsigned)gl.tiles, (unsigned)planes), block(block_dims(gl));
   if constexpr (DIAG) *count = (long long)g.tiles * planes;
   if constexpr (kUsePlanes<L, Real, CT> && !DIAG)
     return launch_pdl(fluid_step_planes_kernel<L, Real, CT, FIRST>, grid, block, 0, s,
-                      planes_of<const Real, L::Q>(cur, g), planes_of<Real, L::Q>(nxt, g), g, omega,
+                      planes_of<const Real, L::Q>(cur, gl), planes_of<Real, L::Q>(nxt, gl), gl, omega,
                       omega_minus);
   else
-    return launch_pdl(fluid_step_kernel<L, Real, CT, DIAG, FIRST>, grid, block, 0, s, cur, nxt, g, omega,
+    return launch_pdl(fluid_step_kernel<L, Real, CT, DIAG, FIRST>, grid, block, 0, s, cur, nxt, gl, omega,
                       omega_minus, partials);
 }
 

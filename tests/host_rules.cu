@@ -1,6 +1,8 @@
 // Test helper: answers questions about the host side of the kernels' launch rules,
 // one per line of standard input, from the engine's own headers.
 //   div n d            n / d through FastDiv
+//   grid nx ny nz      per grid (plain, statistics, FP64 3-D): threads per block, blocks per plane, blocks
+//                      launched; then the partials contract
 //   fluid L OP DIAG nx ny nz    1 if the FP32 fluid step takes two cells per thread
 //   adjoint L OP nx ny nz       the same for the FP32 adjoint step
 //   coupled L FMT RESIDENT nx ny nz    1 if the 16-bit coupled step takes four
@@ -50,13 +52,16 @@ int main() {
     }
     int a[3];
     size_t n[3];
-    const int extra = strcmp(what, "adjoint") == 0 ? 2 : 3;
+    const int extra = strcmp(what, "grid") == 0 ? 0 : strcmp(what, "adjoint") == 0 ? 2 : 3;
     for (int i = 0; i < extra; ++i)
       if (scanf("%d", &a[i]) != 1) return 2;
     if (scanf("%zu %zu %zu", &n[0], &n[1], &n[2]) != 3) return 2;
     Grid g{};
     if (validate_domain(false, 1, 1, 1, n[2] == 1 ? 2 : 3, n[0], n[1], n[2], g) != cudaSuccess) return 3;
-    if (extra == 2) printf("%d\n", a[0] == 9 ? adjoint_of<D2Q9>(a[1], g) : adjoint_of<D3Q19>(a[1], g));
+    if (extra == 0) {
+      for (const Grid& v : {g, stats_grid(g), latency_grid<D3Q19, double>(g, kStepSpread)}) printf("%d %d %lld ", v.bx, v.tiles, v.launched());
+      printf("%lld\n", g.blocks());
+    } else if (extra == 2) printf("%d\n", a[0] == 9 ? adjoint_of<D2Q9>(a[1], g) : adjoint_of<D3Q19>(a[1], g));
     else if (strcmp(what, "fluid") == 0)
       printf("%d\n", a[0] == 9    ? fluid_of<D2Q9>(a[1], a[2], g)
                      : a[0] == 19 ? fluid_of<D3Q19>(a[1], a[2], g)

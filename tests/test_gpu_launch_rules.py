@@ -13,10 +13,11 @@ at boxes that reach them.
   a slot the differences add like independent ones, so the bar is six times 2e-6 of the
   root of the sum of their s^2 (one missing cell, about 1e-2, is 50 times that).
 * FP32 D3Q19 step and diagnostics in the range where the pairs run in 7 or 8 blocks
-  per SM, and of D3Q27, whose diagnostics keep one cell per thread: against the CPU
-  oracle, bit for bit (diagnostics 1e-12).
-* Coupled step with statistics on the kernels with register budgets: against the
-  step without, bit for bit, and the statistics of the fields it wrote, 1e-12."""
+  per SM, of D3Q27, whose diagnostics keep one cell per thread, and of FP64 in small
+  blocks: against the CPU oracle, bit for bit (diagnostics 1e-12).
+* Coupled step with statistics in small blocks and on the kernels with register
+  budgets: against the step without, bit for bit, and the statistics of the fields it
+  wrote, 1e-12."""
 import numpy as np
 import pytest
 import torch
@@ -99,7 +100,9 @@ def test_adjoint_pairs_slot_by_slot(engine, dev, lat, op, dims):
 
 
 STEPS = [("D3Q19", "float", "BGK", (64, 64, 32)), ("D3Q19", "float", "TRT", (52, 50, 54)),
-         ("D3Q19", "float", "MRT", (48, 48, 56)), ("D3Q27", "float", "TRT", (74, 70, 72))]
+         ("D3Q19", "float", "MRT", (48, 48, 56)), ("D3Q27", "float", "TRT", (74, 70, 72)),
+         ("D3Q27", "double", "BGK", (16, 15, 17)), ("D3Q19", "double", "MRT", (7, 9, 11)),
+         ("D3Q19", "double", "RLBM", (33, 2, 5))]
 
 
 @pytest.mark.parametrize("lat,real,op,dims", STEPS)
@@ -120,7 +123,8 @@ def test_steps(engine, dev, lat, real, op, dims):
         assert abs(g - w) <= 1e-12 * max(abs(w), 1e-6)
 
 
-@pytest.mark.parametrize("fl,real,op,dims", [("D3Q27", "double", "TRT", (33, 5, 7)), ("D3Q27", "double", "TRT", (36, 35, 33)),
+@pytest.mark.parametrize("fl,real,op,dims", [("D3Q19", "double", "BGK", (16, 16, 16)), ("D3Q27", "double", "TRT", (33, 5, 7)),
+                                             ("D3Q19", "float", "TRT", (32, 32, 32)), ("D2Q9", "float", "MRT", (64, 63, 1)), ("D3Q27", "double", "TRT", (36, 35, 33)),
                                              ("D2Q9", "float", "TRT", (801, 799, 1))])
 def test_statistics(engine, dev, fl, real, op, dims):
     """The fused statistics against those of the fields it wrote, in scratch of exactly

@@ -3,6 +3,9 @@ the several-cell kernels), compiled from the engine's own headers
 (host_rules.cu) and asked on the host.
 
 * FastDiv equals floor division.
+* Blocks cover every cell of a plane, at most one of them partly, and never more
+  than the partial sums that callers size their scratch by; a small box gets
+  blocks small enough to reach the SMs.
 * Which boxes take several cells per thread. Each expectation is the faster
   kernel of the two as timed on a B200 (the figures stand beside the rules)."""
 import os
@@ -47,6 +50,31 @@ def test_fast_div(ask):
         pairs += [(n, d) for n in sorted(ns)]
     for (n, d), (q,) in zip(pairs, ask([f"div {n} {d}" for n, d in pairs])):
         assert q == n // d, (n, d)
+
+
+def test_blocks_cover_the_plane_within_the_partials(ask):
+    rng = random.Random(7)
+    boxes = [(nx, ny, nz) for nx in (1, 5, 31, 32, 33, 96, 127, 128, 129, 256, 1000) for ny in (1, 2, 7, 64, 300)
+             for nz in (1, 3, 40)]
+    boxes += [tuple(int(2 ** rng.uniform(0, 9)) for _ in range(3)) for _ in range(300)]
+    for (nx, ny, nz), row in zip(boxes, ask(["grid %d %d %d" % b for b in boxes])):
+        assert row[-1] == -(-nx // 128) * ny * nz
+        for bx, tiles, launched in (row[0:3], row[3:6], row[6:9]):
+            where = (nx, ny, nz, bx)
+            assert bx % 32 == 0 and 32 <= bx <= 128, where
+            assert (tiles - 1) * bx < nx * ny <= tiles * bx, where
+            assert launched == tiles * nz <= row[-1], where
+
+
+def test_small_boxes_get_small_blocks(ask):
+    """Threads per block: plain launches, statistics, FP64 launches of a 3-D lattice."""
+    want = {(16, 16, 16): (128, 32, 32), (32, 32, 8): (128, 32, 32), (32, 32, 32): (128, 32, 128), (8, 8, 8): (64, 32, 64),
+            (24, 24, 24): (128, 32, 32), (28, 28, 28): (128, 32, 32), (30, 30, 30): (128, 32, 64), (16, 16, 1): (128, 32, 32), (40, 40, 40): (128, 128, 128),
+            (64, 64, 1): (128, 64, 64),      # the partials of 64-cell rows allow 64
+            (128, 128, 1): (128, 128, 128),  # and those of 128-cell rows 128
+            (64, 64, 32): (128, 128, 128), (256, 256, 256): (128, 128, 128)}
+    got = ask(["grid %d %d %d" % b for b in want])
+    assert {b: (r[0], r[3], r[6]) for b, r in zip(want, got)} == want
 
 
 COUPLED = [
