@@ -181,6 +181,23 @@ __global__ void __launch_bounds__(kThreads, BLOCKS)
     diag_block_to(acc, partials + ((long long)blockIdx.y * gridDim.x + blockIdx.x) * kDiagPartials);
 }
 
+// The blocks of the one-cell step. D2Q9 FP64 BGK (48 registers), where the populations
+// stay in L2 and the launch is past half of the resident blocks: blocks of 96, of
+// which an SM holds 14 (42 warps) where it holds 10 of 128 (40), and which rows of 96
+// and 544 cells fill. 544 x 768 (22 blocks per SM) 6.67 -> 6.48 us, 96 x 4096 6.34 -> 6.07,
+// 512^2 4.68 -> 4.46, 384^2 (7.8) 3.59 -> 3.50; 320^2 (5.4) 3.37 -> 3.41, 800 x 900 (38)
+// 11.9 -> 12.0, 2048^2 91.4 -> 92.4. TRT and MRT level at 544 x 768, 3 % slower at 512^2.
+template <class L, class Real, int CT>
+inline Grid step_grid(const Grid& g) {
+  if (sizeof(Real) == 8 && L::Q == 9 && CT == kBGK && g.launched() > 7LL * kSMs && g.launched() <= 30LL * kSMs) {
+    Grid c = g;
+    c.bx = 96;
+    c.tiles = (int)(((long long)g.nx * g.ny + c.bx - 1) / c.bx);
+    return c;
+  }
+  return latency_grid<L, Real>(g, kStepSpread);
+}
+
 // One step of planes g.z0 .. g.z0 + planes - 1 on the kernel that is the faster one
 // for this lattice, operator, precision and row length. DIAG: with the
 // diagnostics' partials, whose count goes to *count (over every plane; at most
@@ -206,7 +223,7 @@ inline cudaError_t launch_step(const Grid& g, int planes, const Real* cur, Real*
       return run(std::integral_constant<int, kPairBlocks<L, CT>>{});
     }
   }
-  const Grid gl = DIAG || planes != g.nz ? g : latency_grid<L, Real>(g, kStepSpread);
+  const Grid gl = DIAG || planes != g.nz ? g : step_grid<L, Real, CT>(g);
   const dim3 grid((unsigned)gl.tiles, (unsigned)planes), block(block_dims(gl));
   if constexpr (DIAG) *count = (long long)g.tiles * planes;
   if constexpr (kUsePlanes<L, Real, CT> && !DIAG)

@@ -14,7 +14,7 @@ at boxes that reach them.
   root of the sum of their s^2 (one missing cell, about 1e-2, is 50 times that).
 * FP32 D3Q19 step and diagnostics in the range where the pairs run in 7 or 8 blocks
   per SM, of D3Q27, whose diagnostics keep one cell per thread, and of FP64 in small
-  blocks: against the CPU oracle, bit for bit (diagnostics 1e-12).
+  and in 96-thread blocks: against the CPU oracle, bit for bit (diagnostics 1e-12).
 * Coupled step with statistics in small blocks and on the kernels with register
   budgets: against the step without, bit for bit, and the statistics of the fields it
   wrote, 1e-12."""
@@ -102,7 +102,8 @@ def test_adjoint_pairs_slot_by_slot(engine, dev, lat, op, dims):
 STEPS = [("D3Q19", "float", "BGK", (64, 64, 32)), ("D3Q19", "float", "TRT", (52, 50, 54)),
          ("D3Q19", "float", "MRT", (48, 48, 56)), ("D3Q27", "float", "TRT", (74, 70, 72)),
          ("D3Q27", "double", "BGK", (16, 15, 17)), ("D3Q19", "double", "MRT", (7, 9, 11)),
-         ("D3Q19", "double", "RLBM", (33, 2, 5))]
+         ("D3Q19", "double", "RLBM", (33, 2, 5)), ("D2Q9", "double", "BGK", (385, 383, 1)),
+         ("D2Q9", "double", "BGK", (97, 4001, 1)), ("D2Q9", "double", "BGK", (544, 301, 1))]
 
 
 @pytest.mark.parametrize("lat,real,op,dims", STEPS)
