@@ -105,13 +105,14 @@ def build_drivers(force: bool = False) -> list:
     return out
 
 
-CALL = os.path.join(HERE, "_lbcall.so")
+CALL = os.path.join(HERE, "_lbcall" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
 
 
 def build_call(force: bool = False):
     """The native call path of lbcube.py (csrc/pycall.c), an extension module of
-    this Python. Without its headers nothing is built and lbcube.py calls
-    through ctypes."""
+    this Python: its name carries the interpreter's tag, so another one does not
+    find it. Without the Python headers nothing is built and lbcube.py calls through
+    ctypes."""
     inc = sysconfig.get_paths()["include"]
     src = os.path.join(CSRC, "pycall.c")
     if not os.path.exists(os.path.join(inc, "Python.h")):

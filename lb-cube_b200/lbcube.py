@@ -17,6 +17,7 @@ from __future__ import annotations
 import ctypes as C
 import math
 import os
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 # LBCUBE_LIB selects another build of the library (e.g. of an earlier commit, for A/B timing)
@@ -42,7 +43,7 @@ STATS_FIELDS = ("mean_A", "mean_B", "var_A", "var_B", "covariance", "segregation
 
 _lib = None
 _call = None  # the native call path of the step launchers (csrc/pycall.c), or None: ctypes only
-CALL_PATH = os.path.join(HERE, "_lbcall.so")
+CALL_PATH = os.path.join(HERE, "_lbcall" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
 _BLOCK = (16, 8, 1)  # the reference's default block
 
 
@@ -73,7 +74,8 @@ def load() -> C.CDLL:
 
 def _load_call(lib):
     """The extension module that calls the step launchers without ctypes'
-    argument conversion, bound to this library; None where it was not built.
+    argument conversion, bound to this library; None where it was not built for
+    this interpreter (its file name carries the interpreter's tag).
     Its functions return None for arguments other than plain names, ints,
     floats and buffers, which then take the ctypes path."""
     if not os.path.exists(CALL_PATH):
@@ -85,7 +87,7 @@ def _load_call(lib):
         spec = spec_from_file_location("_lbcall", CALL_PATH, loader=ExtensionFileLoader("_lbcall", CALL_PATH))
         mod = module_from_spec(spec)
         spec.loader.exec_module(mod)
-    except ImportError:  # built for another Python
+    except ImportError:
         return None
     mod.setup(*(C.cast(getattr(lib, n), C.c_void_p).value for n in (
         "lbm_step_async", "lbm_step_shifted_async", "lbm_scalar_step_async", "lbm_reaction_ab_async",
