@@ -97,6 +97,7 @@ static int parse_address(PyObject* o, PyObject* attribute, int call, void** out)
   }
   PyObject* v = NULL;
   if (!PyLong_CheckExact(o)) {
+    if (PyLong_Check(o)) return OTHER; /* an int of a class of its own: lbcube.py takes its value */
     v = call ? PyObject_CallMethodNoArgs(o, attribute) : PyObject_GetAttr(o, attribute);
     if (v == NULL) return FAILED;
     o = v;
