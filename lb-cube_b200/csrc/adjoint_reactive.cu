@@ -347,7 +347,7 @@ __global__ void __launch_bounds__(kThreads, kAdjointBlocks<Real>)
 // (native 128^3 gradient 3.13 ms, 3.20 at 5, 3.28 at 6). Each warp adds to the slots of the first
 // of the one-cell blocks that its block covers.
 constexpr int kReactionPairBlocks = 4;
-constexpr CellRule kReactivePairRule{12};
+constexpr CellRule kReactivePairRule{12};  // 24^3 (0.8 blocks per SM) 142 -> 168 us, 64^3 (13.8) 455 -> 442
 
 __device__ __forceinline__ long long pair_warp_slot(const PairGrid& g, int z) {
   return ((long long)z * g.tiles + (long long)kPairCells * blockIdx.x) * kWarpsPerBlock + (long long)(threadIdx.x >> 5);
@@ -1209,7 +1209,7 @@ extern "C" int lbm_reactive_slab_adjoint_unpack_async(int fluid_lattice, int pre
   if (any_overlap(reads, writes)) return (int)cudaErrorInvalidValue;
   const cudaStream_t s = as_stream(stream);
   const long long total = 2LL * g.ny * g.nx;
-  const int blocks = (int)std::min<long long>((total + 255) / 256, 148LL * 16);
+  const int blocks = (int)std::min<long long>((total + 255) / 256, 16LL * kSMs);
   return slab_dispatch(fluid_lattice, precision, LBM_NATIVE, [&](auto fl, auto r, auto) -> int {
     using FL = decltype(fl);
     using R = decltype(r);

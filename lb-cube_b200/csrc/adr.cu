@@ -471,7 +471,7 @@ cudaError_t launch_fluid_reaction_slab_pack(const Real* f, const Real* a, const 
   const Span writes[2] = {{send_lo, hb}, {send_hi, hb}};
   if (any_overlap(reads, writes)) return cudaErrorInvalidValue;
   const long long total = 2LL * g.ny * g.nx;
-  const int blocks = (int)std::min<long long>((total + 255) / 256, 148LL * 16);
+  const int blocks = (int)std::min<long long>((total + 255) / 256, 16LL * kSMs);
   fluid_reaction_slab_pack_kernel<FL, Real><<<blocks, 256, 0, stream>>>(f, a, b, send_lo, send_hi, g);
   return cudaGetLastError();
 }

@@ -85,14 +85,9 @@ __device__ __forceinline__ void warp_sum(double (&v)[N]) {
   }
 }
 
-// Index of this warp's accumulation slot: kThreads / 32 slots per block.
-__device__ __forceinline__ long long warp_slot() {
-  return (long long)block_linear() * (kThreads / 32) + (long long)(threadIdx.x >> 5);
-}
-
-// The same for a launch over some planes of a field (plane_of): blocks indexed
-// by their absolute plane, so launches over different planes of one field use
-// disjoint slots (the same slots as one launch over every plane).
+// Index of this warp's accumulation slot, kThreads / 32 slots per block: blocks
+// indexed by their absolute plane (plane_of), so launches over different planes of
+// one field use disjoint slots (the same slots as one launch over every plane).
 __device__ __forceinline__ long long warp_slot(const Grid& g) {
   return ((long long)plane_of(g) * gridDim.x + blockIdx.x) * (kThreads / 32) +
          (long long)(threadIdx.x >> 5);

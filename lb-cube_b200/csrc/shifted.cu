@@ -229,11 +229,11 @@ cudaError_t launch_convert(int precision, const void* in, void* out, size_t nx, 
   if (any_overlap(reads, writes)) return cudaErrorInvalidValue;
   if (precision == LBM_FLOAT && g.plane % 4 == 0 && (uintptr_t)in % 16 == 0 &&
       (uintptr_t)out % 16 == 0) {
-    const dim3 grid4((unsigned)std::min<long long>((g.plane / 4 + 255) / 256, 148LL * 8),
+    const dim3 grid4((unsigned)std::min<long long>((g.plane / 4 + 255) / 256, 8LL * kSMs),
                      (unsigned)L::Q, 1);
     return launch_pdl(convert4_kernel<L, FMT, ENCODE>, grid4, dim3(256), 0, s, in, out, g.plane, rho0);
   }
-  const dim3 grid((unsigned)std::min<long long>((g.plane + 255) / 256, 148LL * 8), (unsigned)L::Q, 1);
+  const dim3 grid((unsigned)std::min<long long>((g.plane + 255) / 256, 8LL * kSMs), (unsigned)L::Q, 1);
   if (precision == LBM_FLOAT)
     return launch_pdl(convert_kernel<L, FMT, float, ENCODE>, grid, dim3(256), 0, s, in, out, g.plane, rho0);
   return launch_pdl(convert_kernel<L, FMT, double, ENCODE>, grid, dim3(256), 0, s, in, out, g.plane, rho0);

@@ -137,7 +137,7 @@ cudaError_t launch_slab_pack(const Real* f, size_t nx, size_t ny, size_t nz, Rea
   const Span writes[2] = {{send_lo, hbytes}, {send_hi, hbytes}};
   if (any_overlap(reads, writes)) return cudaErrorInvalidValue;
   const long long total = (long long)face_planes<L>() * g.nx * g.ny;
-  const int blocks = (int)std::min<long long>((total + 255) / 256, 148LL * 16);
+  const int blocks = (int)std::min<long long>((total + 255) / 256, 16LL * kSMs);
   slab_pack_kernel<L, Real><<<blocks, 256, 0, s>>>(f, send_lo, send_hi, g.nx, g.ny, g.nz);
   return cudaGetLastError();
 }

@@ -405,8 +405,9 @@ def step_shifted_async(lattice, fmt, collision, cur, nxt, nx, ny, nz, omega, rho
 
 
 def stage_timeouts(reset: bool = False) -> int:
-    """Blocks of the 16-bit step that gave up waiting for their inputs: 0 (the
-    step waits for nothing) once the work launched so far has ended."""
+    """Blocks of the 16-bit step that gave up waiting for their inputs: always 0 (the
+    step waits for nothing). The call waits for the legacy default stream, which
+    does not wait for streams created as non-blocking (torch's side streams)."""
     return int(load().lbm_stage_timeouts(1 if reset else 0))
 
 def encode_shifted_async(lattice, fmt, real, populations, shifted, nx, ny, nz, rho0=1.0,
